@@ -23,8 +23,9 @@
 #include "../../include/parafields_b200.h"
 #include "pf_cg.cuh"
 #include "pf_kernels.cuh"
-#include "pf_fastfft.cuh"
 #include "pf_pairfft.cuh"
+#include "pf_gfft.cuh"
+#include "pf_gfft_plan.hh"
 #include "pf_learned.cuh"
 #include "../include/parafields_b200/fieldio.hh"
 
@@ -173,7 +174,7 @@ static pf_status resolve(const pf_field_desc* d, Geom* g) {
   return PF_OK;
 }
 
-// radix schedule for a pencil length (largest radices first)
+// radix schedule of the passes without device allocation (largest radices first)
 static bool make_radices(int L, Radices* r) {
   r->n = 0;
   int x = L;
@@ -240,7 +241,7 @@ struct pf_plan {
   // learned preconditioner of the residual-mode CG (pf_plan_set_preconditioner), not owned
   pf_learned* learned = nullptr;
   // autotuned choices per generation pass (0 noise, 1 middle c2c, 2 c2r): kernel family
-  // (0: paired FP32 where eligible, 1: scalar) and resident CTAs per SM of persistent
+  // (0: paired FP32 power-of-two kernel where eligible, 1: any-length kernel) and resident CTAs per SM of persistent
   // kernels (0: as many as fit); grid_cap is the value of the pass being launched
   int tune_variant[3] = {0, 0, 0};
   int tune_grid[3] = {0, 0, 0};
@@ -341,90 +342,6 @@ static pf_status tab_put(int dev, int L, int kind, const void* host, size_t byte
   return PF_OK;
 }
 
-template <typename T>
-static pf_status twiddles(pf_plan* P, int L, const cx<T>** out) {
-  if (void* c = tab_find(P->device, L, (int)sizeof(T))) {
-    *out = (const cx<T>*)c;
-    return PF_OK;
-  }
-  std::vector<cx<T>> h(L);
-  for (int m = 0; m < L; m++) {
-    long double a = 2.0L * 3.141592653589793238462643383279502884L * (long double)m / (long double)L;
-    h[m].x = (T)cosl(a);
-    h[m].y = (T)-sinl(a);
-  }
-  void* d = nullptr;
-  TRY(tab_put(P->device, L, (int)sizeof(T), h.data(), sizeof(cx<T>) * (size_t)L, &d));
-  *out = (const cx<T>*)d;
-  return PF_OK;
-}
-
-// Bluestein tables of a length-L transform (layout and definitions in pf_fft.cuh, Blue):
-// one device buffer chirp | bhat | twM, cached in the twiddle map under key (L, 1000+size)
-template <typename T>
-static pf_status blue_tables(pf_plan* P, int L, Blue* out) {
-  int M = 1;
-  while (M < 2 * L - 1) M <<= 1;
-  out->M = M;
-  const int kind = 1000 + (int)sizeof(T);
-  void* d = tab_find(P->device, L, kind);
-  if (!d) {
-    typedef std::complex<double> C;
-    const double pi = 3.141592653589793238462643383279502884;
-    std::vector<C> chirp(L), f(M, C(0, 0)), w(M / 2);
-    for (int j = 0; j < L; j++) {
-      const long long q = ((long long)j * j) % (2LL * L);  // exact phase index
-      chirp[j] = std::polar(1.0, -pi * (double)q / (double)L);
-    }
-    for (int m = 0; m < M / 2; m++) w[m] = std::polar(1.0, -2.0 * pi * (double)m / (double)M);
-    int lg = 0;
-    while ((1 << lg) < M) lg++;
-    auto rev = [&](int i) {
-      int r = 0;
-      for (int k = 0; k < lg; k++) r |= ((i >> k) & 1) << (lg - 1 - k);
-      return r;
-    };
-    // b = conj(chirp) placed circularly, loaded in bit-reversed order for an in-place DIT
-    for (int n = 0; n < L; n++) {
-      f[rev(n)] = std::conj(chirp[n]);
-      if (n > 0) f[rev(M - n)] = std::conj(chirp[n]);
-    }
-    for (int len = 2; len <= M; len <<= 1) {
-      const int step = M / len;
-      for (int i = 0; i < M; i += len)
-        for (int k = 0; k < len / 2; k++) {
-          const C u = f[i + k], v = f[i + k + len / 2] * w[k * step];
-          f[i + k] = u + v;
-          f[i + k + len / 2] = u - v;
-        }
-    }
-    std::vector<cx<T>> h((size_t)L + M + M / 2);
-    for (int j = 0; j < L; j++) h[j] = cx<T>{(T)chirp[j].real(), (T)chirp[j].imag()};
-    for (int m = 0; m < M; m++) {
-      const C v = f[rev(m)] / (double)M;
-      h[L + m] = cx<T>{(T)v.real(), (T)v.imag()};
-    }
-    for (int m = 0; m < M / 2; m++) h[L + M + m] = cx<T>{(T)w[m].real(), (T)w[m].imag()};
-    TRY(tab_put(P->device, L, kind, h.data(), h.size() * sizeof(cx<T>), &d));
-  }
-  const cx<T>* base = (const cx<T>*)d;
-  out->chirp = base;
-  out->bhat = base + L;
-  out->twM = base + L + M;
-  return PF_OK;
-}
-
-// Stockham radices of L, or Bluestein tables (one pencil per tile) when L has a prime
-// factor above 13
-template <typename T>
-static pf_status schedule(pf_plan* P, int L, PassArgs* a) {
-  a->blue = Blue{0, nullptr, nullptr, nullptr};
-  if (make_radices(L, &a->rad)) return PF_OK;
-  if (L > 4096) return fail(PF_ERR_CONFIG, "transform length %d above 4096 has a prime factor above 13", L);
-  a->rad.n = 0;
-  return blue_tables<T>(P, L, &a->blue);
-}
-
 // ---------------------------------------------------------------------------
 // launch helpers
 // ---------------------------------------------------------------------------
@@ -486,79 +403,6 @@ static pf_status set_smem(K kernel, size_t smem) {
   return PF_OK;
 }
 
-// complex pencil pass along a strided axis or along contiguous rows
-template <typename T, bool CONTIG, class Ld, class Mid, class St>
-static pf_status run_pass(pf_plan* P, const char* name, int L, int Lout, long long npencil, long long nouter,
-                          int sign, int sign2, Ld ld, Mid mid, St st, double bytes) {
-  PassArgs a{};
-  a.L = L;
-  a.Lout = Lout;
-  a.npencil = npencil;
-  a.nouter = nouter;
-  a.sign = sign;
-  a.sign2 = sign2;
-  TRY(schedule<T>(P, L, &a));
-  tile_params(L, (int)sizeof(cx<T>), CONTIG, &a);
-  if (a.blue.M) {
-    // Bluestein: one row per tile, or up to 8 interleaved strided pencils (coalesced row
-    // segments) while two CTAs still fit on an SM
-    a.B = 1;
-    if (!CONTIG)
-      while (a.B < 8 && (size_t)2 * a.B * (L + a.blue.M) * sizeof(cx<T>) <= 110 * 1024) a.B *= 2;
-  }
-  const cx<T>* tw = nullptr;
-  TRY(twiddles<T>(P, L, &tw));
-  // Bluestein: the tile buffer plus the M-element scratch (per pencil) in place of the
-  // second buffer
-  const size_t smem = a.blue.M ? ((size_t)(CONTIG ? a.pitch : L) + a.blue.M) * a.B * sizeof(cx<T>)
-                               : smem_of(a, CONTIG, (int)sizeof(cx<T>));
-  if (smem > 227 * 1024) return fail(PF_ERR_CONFIG, "pencil of length %d does not fit in shared memory", L);
-  auto kern = k_pass<T, CONTIG, Ld, Mid, St>;
-  TRY(set_smem(kern, smem));
-  long long grid = CONTIG ? (npencil + a.B - 1) / a.B : ((npencil + a.B - 1) / a.B) * nouter;
-  if (grid <= 0) return PF_OK;
-  ProfRec rec;
-  TRY(prof_begin(P, name, bytes, &rec));
-  kern<<<(unsigned)grid, kThreads, smem, P->stream>>>(a, tw, ld, mid, st);
-  return prof_end(P, &rec);
-}
-
-// real-data passes along dimension 0: rows of T0 = 2L reals <-> L+1 complex
-template <typename T, bool R2C, class Ld, class St>
-static pf_status run_real_pass(pf_plan* P, const char* name, int T0, int Lout, long long rows, Ld ld, St st,
-                               double bytes) {
-  PassArgs a{};
-  a.L = T0 / 2;
-  a.Lout = Lout;
-  a.npencil = rows;
-  a.nouter = 1;
-  a.sign = R2C ? -1 : 1;
-  TRY(schedule<T>(P, a.L, &a));
-  tile_params(a.L, (int)sizeof(cx<T>), true, &a);
-  if (a.blue.M) a.B = 1;
-  const cx<T>* tw = nullptr;
-  const cx<T>* twT = nullptr;
-  TRY(twiddles<T>(P, a.L, &tw));
-  TRY(twiddles<T>(P, T0, &twT));
-  const size_t smem = smem_of(a, true, (int)sizeof(cx<T>)) + (size_t)a.blue.M * sizeof(cx<T>);
-  if (smem > 227 * 1024) return fail(PF_ERR_CONFIG, "row of length %d does not fit in shared memory", T0);
-  long long grid = (rows + a.B - 1) / a.B;
-  if (grid <= 0) return PF_OK;
-  ProfRec rec;
-  if constexpr (R2C) {
-    auto kern = k_r2c<T, Ld, St>;
-    TRY(set_smem(kern, smem));
-    TRY(prof_begin(P, name, bytes, &rec));
-    kern<<<(unsigned)grid, kThreads, smem, P->stream>>>(a, tw, twT, ld, st);
-  } else {
-    auto kern = k_c2r<T, Ld, St>;
-    TRY(set_smem(kern, smem));
-    TRY(prof_begin(P, name, bytes, &rec));
-    kern<<<(unsigned)grid, kThreads, smem, P->stream>>>(a, tw, twT, ld, st);
-  }
-  return prof_end(P, &rec);
-}
-
 // bytes from p to the end of the workspace holding it: the bound every access is checked
 // against (0 for a pointer outside the workspaces)
 static size_t cap_of(const pf_plan* P, const void* p) {
@@ -595,136 +439,7 @@ static pf_status persistent_grid(pf_plan* P, K kern, size_t smem, long long ntil
   return PF_OK;
 }
 
-template <typename T, int SIGN, int SIGN2, class Mid, class St, int L>
-static pf_status launch_fpass_pipe(pf_plan* P, const char* name, int Lout, long long npencil, long long nouter,
-                                   ArrLoad<cx<T>> ld, Mid mid, St st, double bytes) {
-  constexpr int B = fast_B<T, L>();
-  PassArgs a{};
-  a.L = L;
-  a.Lout = Lout;
-  a.B = B;
-  a.npencil = npencil;
-  a.nouter = nouter;
-  const cx<T>* tw = nullptr;
-  TRY(twiddles<T>(P, L, &tw));
-  const size_t smem = fast_smem_pipe<T, L>();
-  auto kern = k_fpass_pipe<T, L, B, SIGN, SIGN2, Mid, St>;
-  TRY(set_smem(kern, smem));
-  const long long ntiles = (npencil + B - 1) / B * nouter;
-  if (ntiles <= 0) return PF_OK;
-  if (npencil > 0x7fffffffLL) return fail(PF_ERR_CONFIG, "pass %s too large", name);
-  unsigned grid = 1;
-  TRY(persistent_grid(P, kern, smem, ntiles, &grid));
-  ProfRec rec;
-  TRY(prof_begin(P, name, bytes, &rec));
-  kern<<<grid, kThreads, smem, P->stream>>>(a, tw, ld, mid, st);
-  return prof_end(P, &rec);
-}
-
-template <typename T, int SIGN, int SIGN2, bool CONTIG, bool PAIR, class Ld, class Mid, class St, int L>
-static pf_status launch_fpass(pf_plan* P, const char* name, int Lout, long long npencil, long long nouter, Ld ld,
-                              Mid mid, St st, double bytes) {
-  if constexpr (!CONTIG && !PAIR && std::is_same<Ld, ArrLoad<cx<T>>>::value)
-    return launch_fpass_pipe<T, SIGN, SIGN2, Mid, St, L>(P, name, Lout, npencil, nouter, ld, mid, st, bytes);
-  constexpr int B = fast_B<T, L>();
-  PassArgs a{};
-  a.L = L;
-  a.Lout = Lout;
-  a.B = B;
-  a.npencil = npencil;
-  a.nouter = nouter;
-  a.sign = SIGN;
-  a.sign2 = SIGN2;
-  const cx<T>* tw = nullptr;
-  TRY(twiddles<T>(P, L, &tw));
-  const size_t smem = fast_smem_pass<T, L>();
-  auto kern = k_fpass<T, L, B, SIGN, SIGN2, CONTIG, PAIR, Ld, Mid, St>;
-  TRY(set_smem(kern, smem));
-  const long long tiles = (npencil + B - 1) / B;
-  const long long grid = CONTIG ? tiles : tiles * nouter;
-  if (grid <= 0) return PF_OK;
-  if (grid > 0x7fffffffLL || npencil > 0x7fffffffLL) return fail(PF_ERR_CONFIG, "pass %s too large", name);
-  ProfRec rec;
-  TRY(prof_begin(P, name, bytes, &rec));
-  kern<<<(unsigned)grid, kThreads, smem, P->stream>>>(a, tw, ld, mid, st);
-  return prof_end(P, &rec);
-}
-
-#define PF_FAST_LENGTHS(X) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536) X(2048)
-
-template <typename T, int SIGN, int SIGN2, bool CONTIG, bool PAIR, class Ld, class Mid, class St>
-static pf_status run_fpass(pf_plan* P, const char* name, int L, int Lout, long long npencil, long long nouter, Ld ld,
-                           Mid mid, St st, double bytes) {
-  switch (L) {
-#define PF_CASE(LL) \
-  case LL:          \
-    return launch_fpass<T, SIGN, SIGN2, CONTIG, PAIR, Ld, Mid, St, LL>(P, name, Lout, npencil, nouter, ld, mid, st, bytes);
-    PF_FAST_LENGTHS(PF_CASE)
-#undef PF_CASE
-    default:
-      return run_pass<T, CONTIG>(P, name, L, Lout, npencil, nouter, SIGN, SIGN2, ld, mid, st, bytes);
-  }
-}
-
-template <typename T, bool R2C, class Ld, class St, int L>
-static pf_status launch_freal(pf_plan* P, const char* name, int Lout, long long rows, Ld ld, St st, double bytes) {
-  constexpr int B = fast_B<T, L>();
-  PassArgs a{};
-  a.L = L;
-  a.Lout = Lout;
-  a.B = B;
-  a.npencil = rows;
-  a.nouter = 1;
-  const cx<T>* tw = nullptr;
-  const cx<T>* twT = nullptr;
-  TRY(twiddles<T>(P, L, &tw));
-  TRY(twiddles<T>(P, 2 * L, &twT));
-  if constexpr (!R2C && std::is_same<Ld, ArrLoad<cx<T>>>::value) {
-    const size_t smemp = fast_smem_real_pipe<T, L>();
-    auto kern = k_fc2r_pipe<T, L, B, St>;
-    TRY(set_smem(kern, smemp));
-    const long long ntiles = (rows + B - 1) / B;
-    if (ntiles <= 0) return PF_OK;
-    if (rows > 0x7fffffffLL) return fail(PF_ERR_CONFIG, "pass %s too large", name);
-    unsigned grid = 1;
-    TRY(persistent_grid(P, kern, smemp, ntiles, &grid));
-    ProfRec rec;
-    TRY(prof_begin(P, name, bytes, &rec));
-    kern<<<grid, kThreads, smemp, P->stream>>>(a, tw, twT, ld, st);
-    return prof_end(P, &rec);
-  }
-  const size_t smem = fast_smem_real<T, L>();
-  const long long grid = (rows + B - 1) / B;
-  if (grid <= 0) return PF_OK;
-  if (grid > 0x7fffffffLL || rows > 0x7fffffffLL) return fail(PF_ERR_CONFIG, "pass %s too large", name);
-  ProfRec rec;
-  if constexpr (R2C) {
-    auto kern = k_fr2c<T, L, B, Ld, St>;
-    TRY(set_smem(kern, smem));
-    TRY(prof_begin(P, name, bytes, &rec));
-    kern<<<(unsigned)grid, kThreads, smem, P->stream>>>(a, tw, twT, ld, st);
-  } else {
-    auto kern = k_fc2r<T, L, B, Ld, St>;
-    TRY(set_smem(kern, smem));
-    TRY(prof_begin(P, name, bytes, &rec));
-    kern<<<(unsigned)grid, kThreads, smem, P->stream>>>(a, tw, twT, ld, st);
-  }
-  return prof_end(P, &rec);
-}
-
-template <typename T, bool R2C, class Ld, class St>
-static pf_status run_freal(pf_plan* P, const char* name, int T0, int Lout, long long rows, Ld ld, St st,
-                           double bytes) {
-  switch (T0 / 2) {
-#define PF_CASE(LL) \
-  case LL:          \
-    return launch_freal<T, R2C, Ld, St, LL>(P, name, Lout, rows, ld, st, bytes);
-    PF_FAST_LENGTHS(PF_CASE)
-#undef PF_CASE
-    default:
-      return run_real_pass<T, R2C>(P, name, T0, Lout, rows, ld, st, bytes);
-  }
-}
+#include "pf_gfft_host.inc"
 
 // row pitch of the half-spectrum work arrays: T0/2+1 rounded up to 8 complex, so every
 // B-wide segment of a strided pass starts on a 64-byte boundary
@@ -740,6 +455,7 @@ static ArrLoad<S> arr_load(const pf_plan* P, const void* p, long long jstride, l
   l.ostride = ostride;
   l.rowstride = rowstride;
   l.Lin = Lin;
+  l.vec = rowstride == 1 && jstride % 2 == 0 && ostride % 2 == 0 && ((uintptr_t)p & 15u) == 0;
   return l;
 }
 
@@ -751,6 +467,7 @@ static ArrStore<S> arr_store(const pf_plan* P, void* p, long long jstride, long 
   s.jstride = jstride;
   s.ostride = ostride;
   s.rowstride = rowstride;
+  s.vec = rowstride == 1 && jstride % 2 == 0 && ostride % 2 == 0 && ((uintptr_t)p & 15u) == 0;
   return s;
 }
 
@@ -927,6 +644,7 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
   TRY(workspace(P, 0, full * sizeof(double2), &A));
   TRY(workspace(P, 1, full * sizeof(double2), &Bw));
   cl.rowmod = g.T[1];
+  cl.mirror = g.mb == PF_MATRIX_DCT;
   if (g.mb == PF_MATRIX_DCT) {
     // Even torus in every dimension (DCT-I, dctmatrixbackend.hh:240-272): the covariance is
     // evaluated only on the prod(T_i/2+1) non-mirrored cells; each later pass reads its
@@ -936,17 +654,17 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
     const long long rows = (long long)D1 * D2;
     cl.rowmod = D1;
     if (vals)
-      TRY((run_freal<double, true>(P, "spec_r2c_vals", g.T[0], T0c, rows,
+      TRY((run_real_pass<double, true>(P, "spec_r2c_vals", g.T[0], T0c, rows,
                                    ValRowLoad{vals, g.T[0], T0c, 1, (unsigned long long)g.D},
                                    arr_store<double2>(P, A, 1, 0, T0c), rows * T0c * 24.0)));
     else
-      TRY((run_freal<double, true>(P, "spec_r2c_cov", g.T[0], T0c, rows, cl, arr_store<double2>(P, A, 1, 0, T0c),
+      TRY((run_real_pass<double, true>(P, "spec_r2c_cov", g.T[0], T0c, rows, cl, arr_store<double2>(P, A, 1, 0, T0c),
                                    rows * T0c * 16.0)));
     spec = (double2*)A;
     if (dim >= 2) {
       MirrorLoad<double2> ml{(const double2*)A, (unsigned)T0c, (unsigned)((long long)T0c * D1), 1u,
                              (unsigned)std::min<size_t>(cap_of(P, A) / sizeof(double2), 0xffffffffu), g.T[1]};
-      TRY((run_fpass<double, -1, -1, false, false>(P, "spec_c2c_d1", g.T[1], D1, T0c, D2, ml, NoMid(),
+      TRY((run_pass<double, false, -1>(P, "spec_c2c_d1", g.T[1], D1, T0c, D2, ml, NoMid(),
                                                    arr_store<double2>(P, Bw, T0c, (long long)T0c * D1, 1),
                                                    (double)T0c * D2 * (D1 + D1) * 16.0)));
       spec = (double2*)Bw;
@@ -954,7 +672,7 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
         const long long inner = (long long)T0c * D1;
         MirrorLoad<double2> m2{(const double2*)Bw, (unsigned)inner, 0u, 1u,
                                (unsigned)std::min<size_t>(cap_of(P, Bw) / sizeof(double2), 0xffffffffu), g.T[2]};
-        TRY((run_fpass<double, -1, -1, false, false>(P, "spec_c2c_d2", g.T[2], D2, inner, 1, m2, NoMid(),
+        TRY((run_pass<double, false, -1>(P, "spec_c2c_d2", g.T[2], D2, inner, 1, m2, NoMid(),
                                                      arr_store<double2>(P, A, inner, 0, 1),
                                                      (double)inner * (D2 + D2) * 16.0)));
         spec = (double2*)A;
@@ -966,17 +684,17 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
     const long long rows = (long long)(g.N / (uint64_t)g.T[0]);
     // dimension 0: covariance evaluation fused into the R2C load
     if (vals)
-      TRY((run_freal<double, true>(P, "spec_r2c_vals", g.T[0], T0c, rows,
+      TRY((run_real_pass<double, true>(P, "spec_r2c_vals", g.T[0], T0c, rows,
                                    ValRowLoad{vals, g.T[0], g.T[0], 0, (unsigned long long)g.N},
                                    arr_store<double2>(P, A, 1, 0, T0c), rows * (T0c * 16.0 + g.T[0] * 8.0))));
     else
-      TRY((run_freal<double, true>(P, "spec_r2c_cov", g.T[0], T0c, rows, cl, arr_store<double2>(P, A, 1, 0, T0c),
+      TRY((run_real_pass<double, true>(P, "spec_r2c_cov", g.T[0], T0c, rows, cl, arr_store<double2>(P, A, 1, 0, T0c),
                                    rows * T0c * 16.0)));
     spec = (double2*)A;
     if (dim >= 2) {
       const int L1 = g.T[1], L1o = dct ? g.T[1] / 2 + 1 : g.T[1];
       const long long outer = dim == 3 ? g.T[2] : 1;
-      TRY((run_fpass<double, -1, -1, false, false>(P, "spec_c2c_d1", L1, L1o, T0c, outer,
+      TRY((run_pass<double, false, -1>(P, "spec_c2c_d1", L1, L1o, T0c, outer,
                                                    arr_load<double2>(P, A, T0c, (long long)T0c * L1, 1, L1), NoMid(),
                                                    arr_store<double2>(P, Bw, T0c, (long long)T0c * L1o, 1),
                                                    (double)T0c * outer * (L1 + L1o) * 16.0)));
@@ -984,7 +702,7 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
       if (dim == 3) {
         const int L2 = g.T[2], L2o = dct ? g.T[2] / 2 + 1 : g.T[2];
         const long long inner = (long long)T0c * L1o;
-        TRY((run_fpass<double, -1, -1, false, false>(P, "spec_c2c_d2", L2, L2o, inner, 1,
+        TRY((run_pass<double, false, -1>(P, "spec_c2c_d2", L2, L2o, inner, 1,
                                                      arr_load<double2>(P, Bw, inner, 0, 1, L2), NoMid(),
                                                      arr_store<double2>(P, A, inner, 0, 1),
                                                      (double)inner * (L2 + L2o) * 16.0)));
@@ -994,11 +712,11 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
   } else {  // DFT matrix: complex torus, every axis complex (dftmatrixbackend.hh:209-238)
     const long long rows = (long long)(g.N / (uint64_t)g.T[0]);
     if (vals)
-      TRY((run_pass<double, true>(P, "spec_c2c_d0", g.T[0], g.T[0], rows, 1, -1, -1,
+      TRY((run_pass<double, true, -1>(P, "spec_c2c_d0", g.T[0], g.T[0], rows, 1,
                                   ValRowLoad{vals, g.T[0], g.T[0], 0, (unsigned long long)g.N}, NoMid(),
                                   arr_store<double2>(P, A, 1, 0, g.T[0]), rows * g.T[0] * 24.0)));
     else
-      TRY((run_pass<double, true>(P, "spec_c2c_d0", g.T[0], g.T[0], rows, 1, -1, -1, cl, NoMid(),
+      TRY((run_pass<double, true, -1>(P, "spec_c2c_d0", g.T[0], g.T[0], rows, 1, cl, NoMid(),
                                   arr_store<double2>(P, A, 1, 0, g.T[0]), rows * g.T[0] * 16.0)));
     spec = (double2*)A;
     void* src = A;
@@ -1007,7 +725,7 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
     for (int ax = 1; ax < dim; ax++) {
       const int L = g.T[ax];
       long long outer = (long long)(g.N / (uint64_t)inner / (uint64_t)L);
-      TRY((run_pass<double, false>(P, ax == 1 ? "spec_c2c_d1" : "spec_c2c_d2", L, L, inner, outer, -1, -1,
+      TRY((run_pass<double, false, -1>(P, ax == 1 ? "spec_c2c_d1" : "spec_c2c_d2", L, L, inner, outer,
                                    arr_load<double2>(P, src, inner, inner * L, 1, L), NoMid(),
                                    arr_store<double2>(P, dst, inner, inner * L, 1), (double)g.N * 32.0)));
       spec = (double2*)dst;
@@ -1161,12 +879,12 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
   if (!(stages & 1)) {
   } else if (F32 && P->tune_variant[0] == 0 && (p2_length(Tl) || p2_length3(Tl)) && p2_view_ok(W1, jst, P0, outer))
     TRY(p2_noise(P, "gen_noise_last", Tl, g.n[last], T0c, outer, nz, p2_store(P, W1, jst, P0, T0c), b1));
-  else if (Tl % 2 == 0)
-    TRY((run_fpass<T, +1, +1, false, true>(P, "gen_noise_last", Tl, g.n[last], T0c, outer, nz, NoMid(),
-                                           arr_store<cx<T>>(P, W1, jst, P0, 1), b1)));
+  else if (noise_dev)
+    TRY((run_pass<T, false, +1>(P, "gen_noise_last", Tl, g.n[last], T0c, outer, R2CNoiseBuf{nz}, NoMid(),
+                                arr_store<cx<T>>(P, W1, jst, P0, 1), b1)));
   else
-    TRY((run_fpass<T, +1, +1, false, false>(P, "gen_noise_last", Tl, g.n[last], T0c, outer, nz, NoMid(),
-                                            arr_store<cx<T>>(P, W1, jst, P0, 1), b1)));
+    TRY((run_pass<T, false, +1>(P, "gen_noise_last", Tl, g.n[last], T0c, outer, nz, NoMid(),
+                                arr_store<cx<T>>(P, W1, jst, P0, 1), b1)));
   if (!(stages & 2)) return PF_OK;
   // the complex-to-real rows of `nrows` (pencil index j1 + n1 * plane) from `src` into
   // the field rows starting at `dst`
@@ -1196,8 +914,9 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
         return p2_c2r(P, "gen_c2r_d0", g.T[0] / 2, g.n[0], nrows, rl, ps, b3);
       }
     }
-    FieldRowStore<S> fr{dst, g.n[0], transform, P->desc.boxcox_lambda, (unsigned)left};
-    return run_freal<T, false>(P, "gen_c2r_d0", g.T[0], g.n[0], nrows,
+    FieldRowStore<S> fr{dst, g.n[0], transform, P->desc.boxcox_lambda, (unsigned)left,
+                        g.n[0] % 2 == 0 && ((uintptr_t)dst % (2 * sizeof(S))) == 0};
+    return run_real_pass<T, false>(P, "gen_c2r_d0", g.T[0], g.n[0], nrows,
                                arr_load<cx<T>>(P, src, 1, 0, P0, T0c), fr, b3);
   };
   if (g.dim == 2) return c2r_rows(W1, out, g.n[1]);
@@ -1223,7 +942,7 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
     else if (p2ok && P->tune_variant[1] != 1)
       TRY(p2_c2c<+1>(P, "gen_c2c_d1", g.T[1], g.n[1], T0c, nz, l1, p2_store(P, W2, P0, w2_plane, T0c), b2));
     else
-      TRY((run_fpass<T, +1, +1, false, false>(P, "gen_c2c_d1", g.T[1], g.n[1], T0c, nz,
+      TRY((run_pass<T, false, +1>(P, "gen_c2c_d1", g.T[1], g.n[1], T0c, nz,
                                               arr_load<cx<T>>(P, src, P0, w1_plane, 1, g.T[1]), NoMid(),
                                               arr_store<cx<T>>(P, W2, P0, w2_plane, 1), b2)));
     TRY(c2r_rows(W2, out + (size_t)g.n[0] * g.n[1] * z0, (long long)g.n[1] * nz));
@@ -1252,26 +971,26 @@ static pf_status gen_dft(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
   SplitStore<S> ss{out, spare, g.n[0], transform, P->desc.boxcox_lambda, (unsigned)g.domain};
   const double e = sizeof(cx<T>);
   if (g.dim == 1) {
-    return run_pass<T, true>(P, "gen_dft_d0", g.T[0], g.n[0], 1, 1, +1, +1, nz, NoMid(), ss,
+    return run_pass<T, true, +1>(P, "gen_dft_d0", g.T[0], g.n[0], 1, 1, nz, NoMid(), ss,
                              (double)g.T[0] * (16.0 + sizeof(T)) + 2.0 * g.n[0] * sizeof(S));
   }
   void *W1 = nullptr, *W2 = nullptr;
   const int last = g.dim - 1;
   const long long inner = (long long)(g.N / (uint64_t)g.T[last]);
   TRY(workspace(P, 0, sizeof(cx<T>) * (size_t)inner * g.n[last], &W1));
-  TRY(run_pass<T, false>(P, "gen_dft_noise", g.T[last], g.n[last], inner, 1, +1, +1, nz, NoMid(),
+  TRY(run_pass<T, false, +1>(P, "gen_dft_noise", g.T[last], g.n[last], inner, 1, nz, NoMid(),
                          arr_store<cx<T>>(P, W1, inner, 0, 1), (double)inner * (g.T[last] * 16.0 + g.n[last] * e)));
   void* cur = W1;
   if (g.dim == 3) {
     TRY(workspace(P, 1, sizeof(cx<T>) * (size_t)g.T[0] * g.n[1] * g.n[2], &W2));
-    TRY((run_pass<T, false>(P, "gen_dft_d1", g.T[1], g.n[1], g.T[0], g.n[2], +1, +1,
+    TRY((run_pass<T, false, +1>(P, "gen_dft_d1", g.T[1], g.n[1], g.T[0], g.n[2],
                             arr_load<cx<T>>(P, W1, g.T[0], (long long)g.T[0] * g.T[1], 1, g.T[1]), NoMid(),
                             arr_store<cx<T>>(P, W2, g.T[0], (long long)g.T[0] * g.n[1], 1),
                             (double)g.T[0] * g.n[2] * (g.T[1] + g.n[1]) * e)));
     cur = W2;
   }
   const long long rows = g.dim == 3 ? (long long)g.n[1] * g.n[2] : g.n[1];
-  return run_pass<T, true>(P, "gen_dft_d0", g.T[0], g.n[0], rows, 1, +1, +1,
+  return run_pass<T, true, +1>(P, "gen_dft_d0", g.T[0], g.n[0], rows, 1,
                            arr_load<cx<T>>(P, cur, 1, 0, g.T[0], g.T[0]), NoMid(), ss,
                            (double)rows * (g.T[0] * e + 2.0 * g.n[0] * sizeof(S)));
 }
@@ -1302,26 +1021,26 @@ static pf_status gen_dctdst(pf_plan* P, const double* noise_dev, uint64_t seed, 
     nz.type = type;
     AccStore<S> as{out, g.n[0], type != 0, (unsigned)g.domain};
     if (g.dim == 1) {
-      TRY(run_pass<T, true>(P, "gen_dctdst_d0", g.T[0], g.n[0], 1, 1, +1, +1, nz, NoMid(), as,
+      TRY(run_pass<T, true, +1>(P, "gen_dctdst_d0", g.T[0], g.n[0], 1, 1, nz, NoMid(), as,
                             (double)g.T[0] * (8.0 + sizeof(T)) + 2.0 * g.n[0] * sizeof(S)));
       continue;
     }
     void *W1 = nullptr, *W2 = nullptr;
     TRY(workspace(P, 0, sizeof(cx<T>) * (size_t)inner * g.n[last], &W1));
-    TRY(run_pass<T, false>(P, "gen_dctdst_noise", g.T[last], g.n[last], inner, 1, +1, +1, nz, NoMid(),
+    TRY(run_pass<T, false, +1>(P, "gen_dctdst_noise", g.T[last], g.n[last], inner, 1, nz, NoMid(),
                            arr_store<cx<T>>(P, W1, inner, 0, 1),
                            (double)inner * (g.T[last] * (8.0 + sizeof(T)) + g.n[last] * e)));
     void* cur = W1;
     if (g.dim == 3) {
       TRY(workspace(P, 1, sizeof(cx<T>) * (size_t)g.T[0] * g.n[1] * g.n[2], &W2));
-      TRY((run_pass<T, false>(P, "gen_dctdst_d1", g.T[1], g.n[1], g.T[0], g.n[2], +1, +1,
+      TRY((run_pass<T, false, +1>(P, "gen_dctdst_d1", g.T[1], g.n[1], g.T[0], g.n[2],
                               arr_load<cx<T>>(P, W1, g.T[0], (long long)g.T[0] * g.T[1], 1, g.T[1]), NoMid(),
                               arr_store<cx<T>>(P, W2, g.T[0], (long long)g.T[0] * g.n[1], 1),
                               (double)g.T[0] * g.n[2] * (g.T[1] + g.n[1]) * e)));
       cur = W2;
     }
     const long long rows = g.dim == 3 ? (long long)g.n[1] * g.n[2] : g.n[1];
-    TRY(run_pass<T, true>(P, "gen_dctdst_d0", g.T[0], g.n[0], rows, 1, +1, +1,
+    TRY(run_pass<T, true, +1>(P, "gen_dctdst_d0", g.T[0], g.n[0], rows, 1,
                           arr_load<cx<T>>(P, cur, 1, 0, g.T[0], g.T[0]), NoMid(), as,
                           (double)rows * (g.T[0] * e + 2.0 * g.n[0] * sizeof(S))));
   }
@@ -1363,8 +1082,10 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
   const int T0c = g.T0c, P0 = half_pitch(g);
   const double e = sizeof(cx<T>);
   const double lb = sizeof(T);
-  FieldRowLoad<S> fl{in, g.n[0], (unsigned)g.domain};
-  FieldRowStore<S> fs{out, g.n[0], 0, 0.0, (unsigned)g.domain};
+  const int row_pairs_in = g.n[0] % 2 == 0 && ((uintptr_t)in % (2 * sizeof(S))) == 0;
+  const int row_pairs_out = g.n[0] % 2 == 0 && ((uintptr_t)out % (2 * sizeof(S))) == 0;
+  FieldRowLoad<S> fl{in, g.n[0], (unsigned)g.domain, row_pairs_in};
+  FieldRowStore<S> fs{out, g.n[0], 0, 0.0, (unsigned)g.domain, row_pairs_out};
   // the real-to-complex and complex-to-real rows along dim 0 take the paired kernels where
   // T0/2 is a power of two in [128, 2048] (FP32 transforms)
   const bool p2rows = std::is_same<T, float>::value && g.T[0] % 2 == 0 && p2_length(g.T[0] / 2);
@@ -1393,7 +1114,7 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
         return p2_r2c(P, "mv_r2c_d0", g.T[0] / 2, nrows, rl, rs, b);
       }
     }
-    return run_freal<T, true>(P, "mv_r2c_d0", g.T[0], T0c, nrows, fl, arr_store<cx<T>>(P, X, 1, 0, P0), b);
+    return run_real_pass<T, true>(P, "mv_r2c_d0", g.T[0], T0c, nrows, fl, arr_store<cx<T>>(P, X, 1, 0, P0), b);
   };
   auto inv_rows = [&](void* X, long long nrows) -> pf_status {
     const double b = (double)nrows * (T0c * e + g.n[0] * sizeof(S));
@@ -1437,7 +1158,7 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
         return p2_c2r(P, "mv_c2r_d0", g.T[0] / 2, g.n[0], nrows, rl, ps, b);
       }
     }
-    return run_freal<T, false>(P, "mv_c2r_d0", g.T[0], g.n[0], nrows, arr_load<cx<T>>(P, X, 1, 0, P0, T0c), fs, b);
+    return run_real_pass<T, false>(P, "mv_c2r_d0", g.T[0], g.n[0], nrows, arr_load<cx<T>>(P, X, 1, 0, P0, T0c), fs, b);
   };
   if (g.dim == 2) {
     void* X1 = nullptr;
@@ -1448,7 +1169,7 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
       TRY(p2_c2c_mid(P, "mv_fused_d1", g.T[1], g.n[1], T0c, 1, p2_load(P, X1, P0, 0, g.n[1], T0c), mid,
                      p2_store(P, X1, P0, 0, T0c), bf1));
     else
-      TRY((run_fpass<T, -1, +1, false, false>(P, "mv_fused_d1", g.T[1], g.n[1], T0c, 1,
+      TRY((run_pass<T, false, -1>(P, "mv_fused_d1", g.T[1], g.n[1], T0c, 1,
                                               arr_load<cx<T>>(P, X1, P0, 0, 1, g.n[1]), mid,
                                               arr_store<cx<T>>(P, X1, P0, 0, 1), bf1)));
     return inv_rows(X1, g.n[1]);
@@ -1469,7 +1190,7 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
     TRY(p2_c2c<-1>(P, "mv_c2c_d1", g.T[1], g.T[1], T0c, g.n[2], p2_load(P, X1, P0, w1o, g.n[1], T0c),
                    p2_store(P, X2, P0, s2, T0c), bd1));
   else
-    TRY((run_fpass<T, -1, -1, false, false>(P, "mv_c2c_d1", g.T[1], g.T[1], T0c, g.n[2],
+    TRY((run_pass<T, false, -1>(P, "mv_c2c_d1", g.T[1], g.T[1], T0c, g.n[2],
                                             arr_load<cx<T>>(P, X1, P0, w1o, 1, g.n[1]), NoMid(),
                                             arr_store<cx<T>>(P, X2, P0, s2, 1), bd1)));
   // forward along dim 2, eigenvalue factor, backward along dim 2 (pencils k0 x k1)
@@ -1478,14 +1199,14 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
     TRY(p2_c2c_mid(P, "mv_fused_d2", g.T[2], g.n[2], T0c, g.T[1], p2_load(P, X2, s2, P0, g.n[2], T0c), mid,
                    p2_store(P, X2, s2, P0, T0c), bf2));
   else
-    TRY((run_fpass<T, -1, +1, false, false>(P, "mv_fused_d2", g.T[2], g.n[2], T0c, g.T[1],
+    TRY((run_pass<T, false, -1>(P, "mv_fused_d2", g.T[2], g.n[2], T0c, g.T[1],
                                             arr_load<cx<T>>(P, X2, s2, P0, 1, g.n[2]), mid,
                                             arr_store<cx<T>>(P, X2, s2, P0, 1), bf2)));
   if (p2d1)
     TRY(p2_c2c<+1>(P, "mv_c2c_d1i", g.T[1], g.n[1], T0c, g.n[2], p2_load(P, X2, P0, s2, g.T[1], T0c),
                    p2_store(P, X1, P0, w1o, T0c), bd1));
   else
-    TRY((run_fpass<T, +1, +1, false, false>(P, "mv_c2c_d1i", g.T[1], g.n[1], T0c, g.n[2],
+    TRY((run_pass<T, false, +1>(P, "mv_c2c_d1i", g.T[1], g.n[1], T0c, g.n[2],
                                             arr_load<cx<T>>(P, X2, P0, s2, 1, g.T[1]), NoMid(),
                                             arr_store<cx<T>>(P, X1, P0, w1o, 1), bd1)));
   return inv_rows(X1, rows);
@@ -1502,37 +1223,37 @@ static pf_status matvec_dft(pf_plan* P, int op, const S* in, S* out) {
   FieldComplexLoad<S> fl{in, g.n[0], (unsigned)g.domain};
   SplitStore<S> ss{out, nullptr, g.n[0], 0, 0.0, (unsigned)g.domain};
   if (g.dim == 1)
-    return run_pass<T, true>(P, "mv_dft_fused_d0", g.T[0], g.n[0], 1, 1, -1, +1, fl, mid, ss,
+    return run_pass<T, true, -1>(P, "mv_dft_fused_d0", g.T[0], g.n[0], 1, 1, fl, mid, ss,
                              (double)g.T[0] * sizeof(T) + 2.0 * g.n[0] * sizeof(S));
   const long long rows = (long long)(g.domain / (uint64_t)g.n[0]);
   void *X1 = nullptr, *X2 = nullptr;
   if (g.dim == 2) {
     TRY(workspace(P, 2, sizeof(cx<T>) * (size_t)g.T[0] * g.n[1], &X1));
-    TRY((run_pass<T, true>(P, "mv_dft_d0", g.T[0], g.T[0], rows, 1, -1, -1, fl, NoMid(),
+    TRY((run_pass<T, true, -1>(P, "mv_dft_d0", g.T[0], g.T[0], rows, 1, fl, NoMid(),
                            arr_store<cx<T>>(P, X1, 1, 0, g.T[0]), (double)rows * (g.n[0] * sizeof(S) + g.T[0] * e))));
-    TRY((run_pass<T, false>(P, "mv_dft_fused_d1", g.T[1], g.n[1], g.T[0], 1, -1, +1,
+    TRY((run_pass<T, false, -1>(P, "mv_dft_fused_d1", g.T[1], g.n[1], g.T[0], 1,
                             arr_load<cx<T>>(P, X1, g.T[0], 0, 1, g.n[1]), mid, arr_store<cx<T>>(P, X1, g.T[0], 0, 1),
                             (double)g.T[0] * 2.0 * g.n[1] * e)));
-    return run_pass<T, true>(P, "mv_dft_d0i", g.T[0], g.n[0], rows, 1, +1, +1,
+    return run_pass<T, true, +1>(P, "mv_dft_d0i", g.T[0], g.n[0], rows, 1,
                              arr_load<cx<T>>(P, X1, 1, 0, g.T[0], g.T[0]), NoMid(), ss,
                              (double)rows * (g.T[0] * e + g.n[0] * sizeof(S)));
   }
   const long long in1 = (long long)g.T[0] * g.T[1];
   TRY(workspace(P, 1, sizeof(cx<T>) * (size_t)g.T[0] * g.n[1] * g.n[2], &X1));
   TRY(workspace(P, 2, sizeof(cx<T>) * (size_t)in1 * g.n[2], &X2));
-  TRY((run_pass<T, true>(P, "mv_dft_d0", g.T[0], g.T[0], rows, 1, -1, -1, fl, NoMid(),
+  TRY((run_pass<T, true, -1>(P, "mv_dft_d0", g.T[0], g.T[0], rows, 1, fl, NoMid(),
                          arr_store<cx<T>>(P, X1, 1, 0, g.T[0]), (double)rows * (g.n[0] * sizeof(S) + g.T[0] * e))));
-  TRY((run_pass<T, false>(P, "mv_dft_d1", g.T[1], g.T[1], g.T[0], g.n[2], -1, -1,
+  TRY((run_pass<T, false, -1>(P, "mv_dft_d1", g.T[1], g.T[1], g.T[0], g.n[2],
                           arr_load<cx<T>>(P, X1, g.T[0], (long long)g.T[0] * g.n[1], 1, g.n[1]), NoMid(),
                           arr_store<cx<T>>(P, X2, g.T[0], in1, 1), (double)g.T[0] * g.n[2] * (g.n[1] + g.T[1]) * e)));
-  TRY((run_pass<T, false>(P, "mv_dft_fused_d2", g.T[2], g.n[2], g.T[0], g.T[1], -1, +1,
+  TRY((run_pass<T, false, -1>(P, "mv_dft_fused_d2", g.T[2], g.n[2], g.T[0], g.T[1],
                           arr_load<cx<T>>(P, X2, in1, g.T[0], 1, g.n[2]), mid, arr_store<cx<T>>(P, X2, in1, g.T[0], 1),
                           (double)in1 * 2.0 * g.n[2] * e)));
-  TRY((run_pass<T, false>(P, "mv_dft_d1i", g.T[1], g.n[1], g.T[0], g.n[2], +1, +1,
+  TRY((run_pass<T, false, +1>(P, "mv_dft_d1i", g.T[1], g.n[1], g.T[0], g.n[2],
                           arr_load<cx<T>>(P, X2, g.T[0], in1, 1, g.T[1]), NoMid(),
                           arr_store<cx<T>>(P, X1, g.T[0], (long long)g.T[0] * g.n[1], 1),
                           (double)g.T[0] * g.n[2] * (g.n[1] + g.T[1]) * e)));
-  return run_pass<T, true>(P, "mv_dft_d0i", g.T[0], g.n[0], rows, 1, +1, +1,
+  return run_pass<T, true, +1>(P, "mv_dft_d0i", g.T[0], g.n[0], rows, 1,
                            arr_load<cx<T>>(P, X1, 1, 0, g.T[0], g.T[0]), NoMid(), ss,
                            (double)rows * (g.T[0] * e + g.n[0] * sizeof(S)));
 }
@@ -1587,15 +1308,11 @@ static pf_status stage_noise(pf_plan* P, const double* noise, int noise_mem, con
 
 template <typename S>
 static pf_status generate_typed(pf_plan* P, const double* nd, uint64_t seed, S* out_dev, int transform) {
-  const bool f64 = sizeof(S) == 8;
-  if (P->g.fb == PF_FIELD_DCTDST)
-    return f64 ? gen_dctdst<double, S>(P, nd, seed, out_dev, transform)
-               : gen_dctdst<float, S>(P, nd, seed, out_dev, transform);
-  if (P->g.fb == PF_FIELD_R2C)
-    return f64 ? gen_r2c<double, S>(P, nd, seed, out_dev, transform) : gen_r2c<float, S>(P, nd, seed, out_dev, transform);
+  // fields of the plan's precision: FP64 transforms for FP64 fields, FP32 for FP32
+  if (P->g.fb == PF_FIELD_DCTDST) return gen_dctdst<S, S>(P, nd, seed, out_dev, transform);
+  if (P->g.fb == PF_FIELD_R2C) return gen_r2c<S, S>(P, nd, seed, out_dev, transform);
   TRY(ensure(P, &P->spare, &P->spare_cap, P->g.domain * sizeof(S)));
-  TRY(f64 ? gen_dft<double, S>(P, nd, seed, out_dev, (S*)P->spare, transform)
-          : gen_dft<float, S>(P, nd, seed, out_dev, (S*)P->spare, transform));
+  TRY((gen_dft<S, S>(P, nd, seed, out_dev, (S*)P->spare, transform)));
   P->spare_valid = true;
   return PF_OK;
 }

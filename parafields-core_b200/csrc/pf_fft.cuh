@@ -1,4 +1,6 @@
-// pf_fft.cuh -- shared-memory Stockham FFT building blocks for sm_100a.
+// pf_fft.cuh -- complex arithmetic, and the shared-memory Stockham transform of the passes that
+// must not allocate device memory (pf_matvec_static); all others are in pf_gfft.cuh and
+// pf_pairfft.cuh.
 //
 // Replaces the FFTW plans of the reference (r2cfieldbackend.hh:210-274,
 // r2cmatrixbackend.hh:254-321, dctmatrixbackend.hh:240-309, dftfieldbackend.hh:186-247).
@@ -248,128 +250,6 @@ __device__ cx<T>* fft_tile(cx<T>* b0, cx<T>* b1, const TileShape& ts, const Radi
     Ns *= R;
   }
   return src;
-}
-
-// ---------------------------------------------------------------------------
-// Bluestein (chirp-z) transform for lengths with a prime factor above 13
-// (L. Bluestein, "A linear filtering approach to the computation of the discrete Fourier
-// transform", 1970): with w_j = exp(s pi i (j^2 mod 2L) / L),
-//   X_k = w_k sum_j (x_j w_j) conj(w_{k-j}),
-// a circular convolution of length M >= 2L-1 (power of two) done in shared memory as an
-// in-place decimation-in-frequency FFT (natural -> bit-reversed order), a pointwise
-// product with the precomputed FFT of conj(w) (bit-reversed order, 1/M folded in), and an
-// in-place decimation-in-time inverse FFT (bit-reversed -> natural order).
-// Tables (sign -1; sign +1 uses their conjugates since conj(w) is symmetric):
-//   chirp[j] = exp(-pi i (j^2 mod 2L)/L), j < L;   bhat[m] = FFT_M(conj chirp)[rev(m)] / M;
-//   twM[m] = exp(-2 pi i m / M), m < M/2.
-// ---------------------------------------------------------------------------
-struct Blue {
-  int M;              // 0: the length is 13-smooth (Stockham stages instead)
-  const void* chirp;  // cx<T>[L]
-  const void* bhat;   // cx<T>[M]
-  const void* twM;    // cx<T>[M/2]
-};
-
-template <typename T>
-__device__ __forceinline__ cx<T> cj_if(cx<T> v, bool c) {
-  if (c) v.y = -v.y;
-  return v;
-}
-
-// in place on the B = 2^lgB pencils of x, element j of pencil b at x[j*B + b] (j < L);
-// work holds M*B elements of shared memory in the same interleaved layout.  M, the
-// butterfly spans and the pencil count are powers of two, so every index is a shift/mask.
-template <typename T>
-__device__ void bluestein(cx<T>* x, cx<T>* work, int L, const Blue& bl, int sign, int lgB = 0) {
-  const int M = bl.M;
-  const int B = 1 << lgB, bm = B - 1;
-  const int lgM = __ffs(M) - 1;
-  const cx<T>* chirp = (const cx<T>*)bl.chirp;
-  const cx<T>* bhat = (const cx<T>*)bl.bhat;
-  const cx<T>* twM = (const cx<T>*)bl.twM;
-  const bool c = sign > 0;
-  for (int u = threadIdx.x; u < (M << lgB); u += blockDim.x) {
-    const int j = u >> lgB;
-    work[u] = j < L ? cmul<T>(x[u], cj_if<T>(__ldg(chirp + j), c)) : mk<T>(0, 0);
-  }
-  __syncthreads();
-  // forward DIF, natural -> bit-reversed; two radix-2 stages (half H, H/2) per pass over
-  // shared memory, a last single stage when log2 M is odd
-  int half = M >> 1, lgh = lgM - 1;
-  for (; half >= 2; half >>= 2, lgh -= 2) {
-    const int q = half >> 1, lgq = lgh - 1;
-    const int lts = lgM - 1 - lgh;  // log2(M / (2 half))
-    for (int u = threadIdx.x; u < ((M >> 2) << lgB); u += blockDim.x) {
-      const int b = u & bm, v = u >> lgB;
-      const int g = v >> lgq, pos = v & (q - 1);
-      const int i0 = g * 2 * half + pos;
-      cx<T>* w0 = work + ((size_t)i0 << lgB) + b;
-      const size_t sq = (size_t)q << lgB, sh = (size_t)half << lgB;
-      cx<T> a0 = w0[0], a1 = w0[sq], a2 = w0[sh], a3 = w0[sh + sq];
-      const cx<T> wA0 = __ldg(twM + (pos << lts)), wA1 = __ldg(twM + ((pos + q) << lts)),
-                  wB = __ldg(twM + (pos << (lts + 1)));
-      cx<T> s0 = cadd<T>(a0, a2), d0 = cmul<T>(csub<T>(a0, a2), wA0);
-      cx<T> s1 = cadd<T>(a1, a3), d1 = cmul<T>(csub<T>(a1, a3), wA1);
-      w0[0] = cadd<T>(s0, s1);
-      w0[sq] = cmul<T>(csub<T>(s0, s1), wB);
-      w0[sh] = cadd<T>(d0, d1);
-      w0[sh + sq] = cmul<T>(csub<T>(d0, d1), wB);
-    }
-    __syncthreads();
-  }
-  if (half == 1) {
-    for (int u = threadIdx.x; u < ((M >> 1) << lgB); u += blockDim.x) {
-      const int b = u & bm, v = u >> lgB;
-      cx<T>* w0 = work + ((size_t)(2 * v) << lgB) + b;
-      const cx<T> a = w0[0], bb = w0[B];
-      w0[0] = cadd<T>(a, bb);
-      w0[B] = csub<T>(a, bb);
-    }
-    __syncthreads();
-  }
-  for (int u = threadIdx.x; u < (M << lgB); u += blockDim.x)
-    work[u] = cmul<T>(work[u], cj_if<T>(__ldg(bhat + (u >> lgB)), c));
-  __syncthreads();
-  // inverse DIT, bit-reversed -> natural; radix-2 stage first when log2 M is odd, then
-  // pairs of stages (half h, 2h)
-  int h = 1, lgh2 = 0;
-  if (lgM & 1) {
-    for (int u = threadIdx.x; u < ((M >> 1) << lgB); u += blockDim.x) {
-      const int b = u & bm, v = u >> lgB;
-      cx<T>* w0 = work + ((size_t)(2 * v) << lgB) + b;
-      const cx<T> a = w0[0], bb = w0[B];
-      w0[0] = cadd<T>(a, bb);
-      w0[B] = csub<T>(a, bb);
-    }
-    __syncthreads();
-    h = 2;
-    lgh2 = 1;
-  }
-  for (; h < M; h <<= 2, lgh2 += 2) {
-    const int ltA = lgM - 1 - lgh2, ltB = lgM - 2 - lgh2;  // log2(M / 2h), log2(M / 4h)
-    for (int u = threadIdx.x; u < ((M >> 2) << lgB); u += blockDim.x) {
-      const int b = u & bm, v = u >> lgB;
-      const int g = v >> lgh2, pos = v & (h - 1);
-      const int i0 = g * 4 * h + pos;
-      cx<T>* w0 = work + ((size_t)i0 << lgB) + b;
-      const size_t s1h = (size_t)h << lgB;
-      const cx<T> wA = conjg<T>(__ldg(twM + (pos << ltA)));
-      const cx<T> wB0 = conjg<T>(__ldg(twM + (pos << ltB))), wB1 = conjg<T>(__ldg(twM + ((pos + h) << ltB)));
-      const cx<T> a0 = w0[0], a1 = cmul<T>(w0[s1h], wA);
-      const cx<T> a2 = w0[2 * s1h], a3 = cmul<T>(w0[3 * s1h], wA);
-      const cx<T> s0 = cadd<T>(a0, a1), d0 = csub<T>(a0, a1);
-      const cx<T> s1 = cadd<T>(a2, a3), d1 = csub<T>(a2, a3);
-      const cx<T> t0 = cmul<T>(s1, wB0), t1 = cmul<T>(d1, wB1);
-      w0[0] = cadd<T>(s0, t0);
-      w0[2 * s1h] = csub<T>(s0, t0);
-      w0[s1h] = cadd<T>(d0, t1);
-      w0[3 * s1h] = csub<T>(d0, t1);
-    }
-    __syncthreads();
-  }
-  for (int u = threadIdx.x; u < (L << lgB); u += blockDim.x)
-    x[u] = cmul<T>(work[u], cj_if<T>(__ldg(chirp + (u >> lgB)), c));
-  __syncthreads();
 }
 
 }  // namespace pf

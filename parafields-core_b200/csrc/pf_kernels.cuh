@@ -40,20 +40,7 @@ struct PassArgs {
   long long nouter;    // strided: outer extent
   int sign, sign2;     // first / second (fused) transform direction
   Radices rad;         // radix schedule of L
-  Blue blue;           // Bluestein tables when L has a prime factor above 13 (then B = 1)
 };
-
-// the 1D transforms of a tile: Stockham stages, or Bluestein (one pencil per tile, unit
-// stride, scratch of blue.M elements after the tile buffers); returns the result buffer
-template <typename T>
-__device__ __forceinline__ cx<T>* fft_any(cx<T>* b0, cx<T>* b1, cx<T>* work, const TileShape& ts, const PassArgs& a,
-                                          const cx<T>* __restrict__ tw, int sign) {
-  if (a.blue.M) {  // strided tiles hold B = 2^k interleaved pencils, row tiles one
-    bluestein<T>(b0, work, a.L, a.blue, sign, ts.bfast ? __ffs(ts.B) - 1 : 0);
-    return b0;
-  }
-  return fft_tile<T>(b0, b1, ts, a.rad, tw, sign);
-}
 
 struct NoMid {
   static constexpr bool active = false;
@@ -62,13 +49,6 @@ struct NoMid {
     return v;
   }
 };
-
-// loaders that produce elements j and j + L/2 of a pencil from one generator call
-struct R2CNoise;
-template <class Ld>
-struct has_pair_load : std::false_type {};
-template <>
-struct has_pair_load<R2CNoise> : std::true_type {};
 
 // Generic complex pencil pass.  CONTIG: pencils are rows (element j of row p at
 // stride 1); otherwise pencil p of outer block o has element j at p + j*jstride +
@@ -102,30 +82,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pass(const PassArgs a, const cx
     p0 = (blockIdx.x - io * tpo) * a.B;
   }
   const int tot = a.B * a.L;
-  bool loaded = false;
-  if constexpr (has_pair_load<Ld>::value) {
-    if (a.L % 2 == 0) {  // one generator call for elements j and j + L/2
-      const int h = a.L / 2;
-      for (int u = threadIdx.x; u < a.B * h; u += blockDim.x) {
-        int b, j;
-        if (CONTIG) {
-          b = u / h;
-          j = u - b * h;
-        } else {
-          b = u % a.B;
-          j = u / a.B;
-        }
-        const long long p = p0 + b;
-        cx<T> v0 = mk<T>(0, 0), v1 = mk<T>(0, 0);
-        if (p < a.npencil) ld.template load2<T>((int)p, j, (int)io, v0, v1);
-        b0[b * ts.sb + j * ts.sj] = v0;
-        b0[b * ts.sb + (j + h) * ts.sj] = v1;
-      }
-      loaded = true;
-    }
-  }
-  if (!loaded)
-    for (int u = threadIdx.x; u < tot; u += blockDim.x) {
+  for (int u = threadIdx.x; u < tot; u += blockDim.x) {
       int b, j;
       if (CONTIG) {
         b = u / a.L;
@@ -138,8 +95,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pass(const PassArgs a, const cx
       b0[b * ts.sb + j * ts.sj] = (p < a.npencil) ? ld.template load<T>(p, j, io) : mk<T>(0, 0);
     }
   __syncthreads();
-  cx<T>* wk = b1;  // Bluestein scratch (b1 is not used as a Stockham buffer then)
-  cx<T>* r = fft_any<T>(b0, b1, wk, ts, a, tw, a.sign);
+  cx<T>* r = fft_tile<T>(b0, b1, ts, a.rad, tw, a.sign);
   if (Mid::active) {
     for (int u = threadIdx.x; u < tot; u += blockDim.x) {
       int b, j;
@@ -154,7 +110,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pass(const PassArgs a, const cx
       if (p < a.npencil) r[b * ts.sb + j * ts.sj] = mid.template operator()<T>(p, j, io, r[b * ts.sb + j * ts.sj]);
     }
     __syncthreads();
-    r = fft_any<T>(r, r == b0 ? b1 : b0, wk, ts, a, tw, a.sign2);
+    r = fft_tile<T>(r, r == b0 ? b1 : b0, ts, a.rad, tw, a.sign2);
   }
   const int tout = a.B * a.Lout;
   for (int u = threadIdx.x; u < tout; u += blockDim.x) {
@@ -192,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_r2c(const PassArgs a, const cx<
     b0[b * a.pitch + m] = z;
   }
   __syncthreads();
-  cx<T>* Z = fft_any<T>(b0, b1, b1 + a.B * a.pitch, ts, a, tw, -1);
+  cx<T>* Z = fft_tile<T>(b0, b1, ts, a.rad, tw, -1);
   cx<T>* X = (Z == b0) ? b1 : b0;
   const int L = a.L;
   for (int u = threadIdx.x; u < a.B * (L + 1); u += blockDim.x) {
@@ -245,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_c2r(const PassArgs a, const cx<
     b0[b * a.pitch + k] = mk<T>(s.x - t.y, s.y + t.x);  // s + i t
   }
   __syncthreads();
-  cx<T>* z = fft_any<T>(b0, b1, b1 + a.B * a.pitch, ts, a, tw, +1);
+  cx<T>* z = fft_tile<T>(b0, b1, ts, a.rad, tw, +1);
   for (int u = threadIdx.x; u < a.B * a.Lout; u += blockDim.x) {
     const int b = u / a.Lout, j = u - b * a.Lout;
     const long long p = p0 + b;
@@ -265,6 +221,7 @@ struct ArrLoad {
   unsigned jstride, ostride, rowstride;
   unsigned n;  // elements in the buffer
   int Lin;     // j >= Lin reads zero (input pruning / zero padding)
+  int vec;     // pencils adjacent, even strides, 16-byte aligned: two FP32 pencils per load
   template <typename T>
   __device__ __forceinline__ cx<T> load(long long p, int j, long long o) const {
     if (j >= Lin) return mk<T>(0, 0);
@@ -298,6 +255,7 @@ struct ArrStore {
   S* ptr;
   unsigned jstride, ostride, rowstride;
   unsigned n;
+  int vec;  // as in ArrLoad
   template <typename T>
   __device__ __forceinline__ void store(long long p, int j, long long o, cx<T> v) const {
     const unsigned i = (unsigned)p * rowstride + (unsigned)j * jstride + (unsigned)o * ostride;
@@ -327,9 +285,27 @@ __device__ __forceinline__ T apply_mutator(int kind, T lam, T v) {
 // r2cfieldbackend.hh:352-368): row p holds x[p*n0 + j] for j < n0, zero beyond
 template <typename S>
 struct FieldRowLoad {
+  using S2 = typename std::conditional<sizeof(S) == 8, double2, float2>::type;
   const S* x;
   int n0;
   unsigned n;
+  int vec;  // n0 even and x aligned for pairs
+  // reals 2m and 2m + 1
+  template <typename T>
+  __device__ __forceinline__ void real2(int p, int m, T& a, T& b) const {
+    if (vec) {
+      const unsigned i = (unsigned)p * (unsigned)n0 + 2u * (unsigned)m;
+      a = b = (T)0;
+      if (2 * m < n0 && in_bounds32(i + 1, n)) {
+        const S2 v = *reinterpret_cast<const S2*>(x + i);
+        a = (T)v.x;
+        b = (T)v.y;
+      }
+      return;
+    }
+    a = real<T>(p, 2 * m);
+    b = real<T>(p, 2 * m + 1);
+  }
   template <typename T>
   __device__ __forceinline__ T real(long long p, int j) const {
     if (j >= n0) return (T)0;
@@ -342,11 +318,32 @@ struct FieldRowLoad {
 // r2cfieldbackend.hh:433-441) with an optional value transform
 template <typename S>
 struct FieldRowStore {
+  using S2 = typename std::conditional<sizeof(S) == 8, double2, float2>::type;
   S* out;
   int n0;
   int transform;
   double boxcox;
   unsigned n;
+  int vec;  // n0 even and out aligned for pairs
+  // reals 2m and (when `two`) 2m + 1
+  template <typename T>
+  __device__ __forceinline__ void real2(int p, int m, T a, T b, bool two) const {
+    if (vec && two) {
+      if (transform) {
+        a = apply_mutator<T>(transform, (T)boxcox, a);
+        b = apply_mutator<T>(transform, (T)boxcox, b);
+      }
+      const unsigned i = (unsigned)p * (unsigned)n0 + 2u * (unsigned)m;
+      if (!in_bounds32(i + 1, n)) return;
+      S2 v;
+      v.x = (S)a;
+      v.y = (S)b;
+      *reinterpret_cast<S2*>(out + i) = v;
+      return;
+    }
+    real<T>(p, 2 * m, a);
+    if (two) real<T>(p, 2 * m + 1, b);
+  }
   template <typename T>
   __device__ __forceinline__ void real(long long p, int j, T v) const {
     if (transform) v = apply_mutator<T>(transform, (T)boxcox, v);
@@ -533,11 +530,16 @@ __device__ inline double bessel_k(double nu, double x) {
   return km;
 }
 
+// products and sums of the covariance's arguments are rounded one by one, as the reference
+// computes them: contracted to fused multiply-adds (which depends on what the compiler inlines)
+// they move small eigenvalues by up to 1e-12 of their value
+__device__ __forceinline__ double cov_madd(double a, double b, double s) { return __dadd_rn(s, __dmul_rn(a, b)); }
+
 __device__ __forceinline__ double cov_eval(const CovParams& c, const double* xt) {
   const double var = c.variance;
   const int dim = c.dim;
   double sum = 0.;
-  for (int i = 0; i < dim; i++) sum += xt[i] * xt[i];
+  for (int i = 0; i < dim; i++) sum = cov_madd(xt[i], xt[i], sum);
   switch (c.cov) {
     case 2: {  // spherical, covariance.hh:310-340
       const double h = sqrt(sum);
@@ -560,11 +562,11 @@ __device__ __forceinline__ double cov_eval(const CovParams& c, const double* xt)
     }
     case 5: {  // matern32
       const double h = sqrt(sum);
-      return var * (1. + sqrt(3.) * h) * exp(-sqrt(3.) * h);
+      return var * cov_madd(sqrt(3.), h, 1.) * exp(-sqrt(3.) * h);
     }
     case 6: {  // matern52
       const double h = sqrt(sum);
-      return var * (1. + sqrt(5.) * h + 5. / 3. * h * h) * exp(-sqrt(5.) * h);
+      return var * cov_madd(5. / 3. * h, h, cov_madd(sqrt(5.), h, 1.)) * exp(-sqrt(5.) * h);
     }
     case 7: {  // dampedOscillation
       const double h = sqrt(sum);
@@ -606,7 +608,7 @@ __device__ __forceinline__ void geo_apply(const CovParams& c, const double* x, d
   } else {
     for (int i = 0; i < c.dim; i++) {
       double s = 0.;
-      for (int k = 0; k < c.dim; k++) s += c.geo[i * c.dim + k] * x[k];
+      for (int k = 0; k < c.dim; k++) s = cov_madd(c.geo[i * c.dim + k], x[k], s);
       xt[i] = s;
     }
   }
@@ -738,8 +740,8 @@ __device__ __noinline__ double cofold_integral(const CovParams& c, double alpha,
 // classical coordinates of torus cell jj (computeMatrixEntriesWithMirroring, matrix.hh:615-638)
 __device__ __forceinline__ void classical_coord(const CovParams& c, const int* jj, double* x) {
   for (int i = 0; i < c.dim; i++) {
-    double v = (double)(unsigned int)jj[i] * c.h[i];
-    if (v > c.half[i]) v -= c.wrap[i];
+    double v = __dmul_rn((double)(unsigned int)jj[i], c.h[i]);
+    if (v > c.half[i]) v = __dsub_rn(v, c.wrap[i]);
     x[i] = v;
   }
 }
@@ -764,7 +766,7 @@ __device__ __forceinline__ double cov_classical(const CovParams& c, const double
   } else {
     for (int i = 0; i < c.dim; i++) {
       double s = 0.;
-      for (int k = 0; k < c.dim; k++) s += c.geo[i * c.dim + k] * x[k];
+      for (int k = 0; k < c.dim; k++) s = cov_madd(c.geo[i * c.dim + k], x[k], s);
       xt[i] = s;
     }
   }
@@ -800,10 +802,17 @@ struct CovRowLoad {
   CovParams c;
   int rowmod;  // rows enumerate (j1, j2) with j1 = p % rowmod (T1 for the full torus,
                // T1/2+1 when only the non-mirrored rows of an even torus are needed)
+  int mirror;  // rows even about T0/2 (DCT matrix): cells beyond it repeat those before it
+  template <typename T>
+  __device__ __forceinline__ void real2(int p, int m, T& a, T& b) const {
+    a = real<T>(p, 2 * m);
+    b = real<T>(p, 2 * m + 1);
+  }
   template <typename T>
   __device__ __forceinline__ T real(long long p, int j) const {
-    const int j1 = c.dim > 1 ? (int)(p % rowmod) : 0;
-    const int j2 = c.dim > 2 ? (int)(p / rowmod) : 0;
+    const unsigned q = (unsigned)p;
+    const int j1 = c.dim > 1 ? (int)(q % (unsigned)rowmod) : 0;
+    const int j2 = c.dim > 2 ? (int)(q / (unsigned)rowmod) : 0;
     return (T)cov_at(c, j, j1, j2);
   }
   template <typename T>
@@ -822,6 +831,11 @@ struct ValRowLoad {
   int rowlen;
   int mirror;
   unsigned long long n;
+  template <typename T>
+  __device__ __forceinline__ void real2(int p, int m, T& a, T& b) const {
+    a = real<T>(p, 2 * m);
+    b = real<T>(p, 2 * m + 1);
+  }
   template <typename T>
   __device__ __forceinline__ T real(long long p, int j) const {
     const int jj = (mirror && j > T0 / 2) ? T0 - j : j;
@@ -992,29 +1006,11 @@ struct R2CNoise {
     }
     return scale<T>(k0, k1, j, r1, r2);
   }
-  // elements j and j + L/2 from one generator call (L even, no noise buffer)
-  template <typename T>
-  __device__ __forceinline__ void load2(int pl, int j, int io, cx<T>& v0, cx<T>& v1) const {
-    int k0, k1;
-    decode(pl, io, k0, k1);
-    const int h = Tl / 2;
-    T r1, r2, r3, r4;
-    if (noise) {
-      const unsigned s0 = stored(k0, k1, j), s1 = stored(k0, k1, j + h);
-      if (!in_bounds32(2 * s0 + 1, nnoise) || !in_bounds32(2 * s1 + 1, nnoise)) return;
-      r1 = (T)noise[2 * s0];
-      r2 = (T)noise[2 * s0 + 1];
-      r3 = (T)noise[2 * s1];
-      r4 = (T)noise[2 * s1 + 1];
-    } else {
-      const uint4 c = pair_bits(seed, stored(k0, k1, j), epoch ? __ldg(epoch) : 0u);
-      box_muller(c.x, c.y, r1, r2);
-      box_muller(c.z, c.w, r3, r4);
-    }
-    v0 = scale<T>(k0, k1, j, r1, r2);
-    v1 = scale<T>(k0, k1, j + h, r3, r4);
-  }
 };
+
+// R2CNoise whose normals come from a buffer in the reference's draw order: no arithmetic worth
+// staging, so the passes load it straight into their first stage
+struct R2CNoiseBuf : R2CNoise {};
 
 // full-torus complex noise of the DFT backend (dftfieldbackend.hh:276-280); the pass
 // runs along the slowest dimension d-1 first (contiguous when dim == 1)

@@ -20,11 +20,14 @@
 #include <cuda.h>
 
 #include "pf_cg.cuh"
-#include "pf_fastfft.cuh"
+#include "pf_kernels.cuh"
 
 namespace pf {
 
 constexpr int kP2Threads = 256;
+
+// radix of the next Stockham stage of m remaining points
+constexpr int pick_radix(int m) { return m % 8 == 0 ? 8 : (m % 4 == 0 ? 4 : 2); }
 // resident CTAs per SM the register allocation is sized for (per kernel family).  The
 // strided pass is held to 64 registers (4 CTAs per SM): alone it runs as fast as with 3,
 // and in the two-stream batch its CTAs fit beside the other stream's kernels (256^3
