@@ -275,6 +275,9 @@ struct pf_plan {
   // residual-mode CG: the same matvec's last pass also sums cg_dot_d . out into *cg_dot_dst
   const double* cg_dot_d = nullptr;
   double* cg_dot_dst = nullptr;
+  // kernels may start while their predecessor in the stream drains (launch_chained); off while
+  // two streams of a batch share the SMs, where waiting blocks would hold the other's places
+  bool chain = true;
 };
 
 static pf_status dalloc(pf_plan* P, void** p, size_t bytes) {
@@ -372,6 +375,23 @@ static pf_status prof_end(pf_plan* P, ProfRec* rec) {
   CK(cudaEventRecord(rec->e1, P->stream));
   P->recs.push_back(*rec);
   return PF_OK;
+}
+
+// launch on the plan's stream that may start while the kernel before it in the stream drains
+// (chain_start / chain_wait in pf_cg.cuh); for kernels that call both
+template <class... K, class... A>
+static void launch_chained(pf_plan* P, void (*kern)(K...), unsigned grid, unsigned block, size_t smem, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = P->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = P->chain ? 1 : 0;
+  (void)cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);  // errors: cudaGetLastError in prof_end
 }
 
 static int pow2_floor(int x) {
@@ -633,8 +653,8 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
     unsigned long long* keys = (unsigned long long*)P->cof;
     ProfRec rec;
     TRY(prof_begin(P, "spec_cofold_stats", 0.0, &rec));
-    k_cofold_stats<<<grid_for((uint64_t)C[0] * C[1] * C[2]), kThreads, 0, P->stream>>>(sc, C[0], C[1], C[2], keys);
-    k_cofold_finish<<<1, 32, 0, P->stream>>>(sc, d->cofold_max_factor, keys, P->cof + 2);
+    launch_chained(P, k_cofold_stats, grid_for((uint64_t)C[0] * C[1] * C[2]), kThreads, 0, sc, C[0], C[1], C[2], keys);
+    launch_chained(P, k_cofold_finish, 1, 32, 0, sc, d->cofold_max_factor, keys, P->cof + 2);
     TRY(prof_end(P, &rec));
     cl.c.cof = P->cof + 2;
   }
@@ -756,7 +776,7 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
   {
     ProfRec rec;
     TRY(prof_begin(P, "spec_scan", g.S * (16.0 + 24.0), &rec));
-    k_scan<<<grid_for(g.S), kThreads, 0, P->stream>>>(sa);
+    launch_chained(P, k_scan, grid_for(g.S), kThreads, 0, sa);
     TRY(prof_end(P, &rec));
   }
   ScanOut so;
@@ -818,7 +838,7 @@ static pf_status factor_array(pf_plan* P, int op, const T** out) {
     TRY(dalloc(P, &P->fac[a][op], P->g.S * sizeof(T)));
     ProfRec rec;
     TRY(prof_begin(P, "factors", P->g.S * (8.0 + sizeof(T)), &rec));
-    k_factors<T><<<grid_for(P->g.S), kThreads, 0, P->stream>>>(P->lam64, P->g.S, 1.0 / (double)P->g.N, op,
+    launch_chained(P, k_factors<T>, grid_for(P->g.S), kThreads, 0, P->lam64, P->g.S, 1.0 / (double)P->g.N, op,
                                                                (T*)P->fac[a][op]);
     TRY(prof_end(P, &rec));
   }
@@ -1047,7 +1067,7 @@ static pf_status gen_dctdst(pf_plan* P, const double* noise_dev, uint64_t seed, 
   if (transform) {  // the value transform acts on the summed field (randomfield.hh:641-651)
     ProfRec rec;
     TRY(prof_begin(P, "transform", g.domain * 2.0 * sizeof(S), &rec));
-    k_transform<S><<<grid_for(g.domain), kThreads, 0, P->stream>>>(out, g.domain, transform, P->desc.boxcox_lambda);
+    launch_chained(P, k_transform<S>, grid_for(g.domain), kThreads, 0, out, g.domain, transform, P->desc.boxcox_lambda);
     TRY(prof_end(P, &rec));
   }
   return PF_OK;
@@ -1337,6 +1357,7 @@ static pf_status generate_stage_pipeline(pf_plan* P, uint64_t seed, int32_t coun
   cudaEvent_t* noise_done = P->stage_ev;      // [slot]: the noise pass wrote the buffer
   cudaEvent_t* buffer_free = P->stage_ev + 2;  // [slot]: the remaining passes read it
   pf_status st = PF_OK;
+  P->chain = false;
   for (int32_t r = 0; r < count && st == PF_OK; r++) {
     const int slot = r & 1;
     auto run = [&](int stages) {
@@ -1370,6 +1391,7 @@ static pf_status generate_stage_pipeline(pf_plan* P, uint64_t seed, int32_t coun
     P->stream = caller;
   }
   P->stream = caller;
+  P->chain = true;
   for (int l = 0; l < 2; l++) {
     CK(cudaEventRecord(P->lane_ev[1 + l], P->lane[l]));
     CK(cudaStreamWaitEvent(caller, P->lane_ev[1 + l], 0));
@@ -1630,6 +1652,7 @@ pf_status pf_generate_batch(pf_plan* P, uint64_t seed, int32_t count, void* out,
       TRY(ensure(P, &P->io2_dev, &P->io2_cap, bytes));
     }
     pf_status st = PF_OK;
+    P->chain = false;
     for (int32_t r = 0; r < count && st == PF_OK; r++) {
       const int slot = r & 1;
       void* dst = host ? (slot ? P->io2_dev : P->io_dev) : (char*)out + (size_t)r * bytes;
@@ -1654,6 +1677,7 @@ pf_status pf_generate_batch(pf_plan* P, uint64_t seed, int32_t count, void* out,
           std::swap(P->ws_bytes[i], P->ws_b_bytes[i]);
         }
     }
+    P->chain = true;
     for (int l = 0; l < 2; l++) {
       CK(cudaEventRecord(P->lane_ev[1 + l], P->lane[l]));
       CK(cudaStreamWaitEvent(caller, P->lane_ev[1 + l], 0));
@@ -1783,7 +1807,7 @@ pf_status pf_export_noise(pf_plan* P, uint64_t seed, uint32_t epoch, double* out
     TRY(ensure(P, (void**)&P->noise_dev, &P->noise_cap, g.noise * 8));
     dst = P->noise_dev;
   }
-  k_export_noise<<<grid_for(g.Nc), kThreads, 0, P->stream>>>(e, dst);
+  launch_chained(P, k_export_noise, grid_for(g.Nc), kThreads, 0, e, dst);
   P->launches++;
   CK(cudaGetLastError());
   if (mem != PF_MEM_DEVICE) CK(cudaMemcpyAsync(out, dst, g.noise * 8, cudaMemcpyDeviceToHost, P->stream));
@@ -1802,10 +1826,10 @@ pf_status pf_apply_transform(pf_plan* P, int32_t precision, void* data, uint64_t
   ProfRec rec;
   TRY(prof_begin(P, "transform", count * 2.0 * es, &rec));
   if (es == 8)
-    k_transform<double><<<grid_for(count), kThreads, 0, P->stream>>>((double*)d, count, P->desc.transform,
+    launch_chained(P, k_transform<double>, grid_for(count), kThreads, 0, (double*)d, count, P->desc.transform,
                                                                     P->desc.boxcox_lambda);
   else
-    k_transform<float><<<grid_for(count), kThreads, 0, P->stream>>>((float*)d, count, P->desc.transform,
+    launch_chained(P, k_transform<float>, grid_for(count), kThreads, 0, (float*)d, count, P->desc.transform,
                                                                    P->desc.boxcox_lambda);
   TRY(prof_end(P, &rec));
   if (mem != PF_MEM_DEVICE) CK(cudaMemcpyAsync(data, d, count * es, cudaMemcpyDeviceToHost, P->stream));

@@ -913,6 +913,8 @@ template <typename T, bool ROWS, int MODE, int SIGN, bool FUSED, class Ld, class
 __global__ void __launch_bounds__(kGThreads, 1)
     k_g(const __grid_constant__ GArgs<T> a, const __grid_constant__ Ld ld, const __grid_constant__ Mid mid,
         const __grid_constant__ St st) {
+  chain_start();
+  chain_wait();
   using R_ = typename GT<T>::R;
   using V = CV<R_>;
   constexpr int PAIR = GT<T>::PAIR;

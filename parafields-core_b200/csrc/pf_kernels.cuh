@@ -3,6 +3,7 @@
 
 #include <math.h>
 
+#include "pf_cg.cuh"
 #include "pf_fft.cuh"
 
 namespace pf {
@@ -1302,6 +1303,8 @@ __device__ __forceinline__ void scan_one(double v, double thr, unsigned int& sm,
 }
 
 __global__ void __launch_bounds__(kThreads) k_scan(const ScanArgs a) {
+  chain_start();
+  chain_wait();
   unsigned int sm = 0, ze = 0, ne = 0;
   double mn = 1.7976931348623157e308;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -1372,6 +1375,8 @@ __global__ void __launch_bounds__(kThreads) k_scan(const ScanArgs a) {
 // factor arrays for the matvecs: lambda/N, sqrt(lambda)/N, 1/(lambda N), pinv(lambda)/N
 template <typename T>
 __global__ void k_factors(const double* __restrict__ lam, uint64_t n, double invN, int op, T* out) {
+  chain_start();
+  chain_wait();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const double l = lam[i];
     double f;
@@ -1389,6 +1394,8 @@ __global__ void k_factors(const double* __restrict__ lam, uint64_t n, double inv
 
 template <typename S>
 __global__ void k_transform(S* v, uint64_t n, int kind, double lam) {
+  chain_start();
+  chain_wait();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
     v[i] = apply_mutator<S>(kind, (S)lam, v[i]);
 }

@@ -397,6 +397,8 @@ struct NoiseExport {
 };
 
 __global__ void k_export_noise(NoiseExport e, double* __restrict__ out) {
+  chain_start();
+  chain_wait();
   const bool paired = e.Tl % 2 == 0;
   const int kls = paired ? e.Tl / 2 : e.Tl;
   const int n1 = e.dim == 3 ? e.ext1 : 1;
@@ -612,21 +614,27 @@ struct P2Noise {
   }
 };
 
-// Tile order of the persistent passes.  With a counter (zeroed in the stream before the
-// launch) every CTA takes its next tile index from it, so CTAs on SMs that run faster take
-// more tiles and the launch ends when the work does (the noise pass alone: 0.263 against 0.284
-// ms with the static order on the 256^3 workload).  Thread 0 fetches the index of the next
-// tile while the current one is transformed; the other threads read it after the barrier at
-// the end of the tile (every tile body passes barriers after the previous read of *s).
-// Without a counter the CTAs stride over the tiles by the grid size.
-__device__ __forceinline__ long long tile_first(unsigned long long* ctr, long long* s) {
+// Tile order of the persistent passes.  With a counter (0 between launches) every CTA takes its
+// next tile index from it, so CTAs on SMs that run faster take more tiles and the launch ends
+// when the work does (the noise pass alone: 0.263 against 0.284 ms with the static order on the
+// 256^3 workload).  Thread 0 fetches the index of the next tile while the current one is
+// transformed; the other threads read it after the barrier at the end of the tile (every tile
+// body passes barriers after the previous read of *s).  Each CTA fetches once more than it has
+// tiles, ntiles + gridDim.x fetches in all; the last one resets the counter, so no memset (2 us
+// of the stream) precedes a launch.  Without a counter the CTAs stride over the tiles by the grid size.
+__device__ __forceinline__ unsigned long long tile_take(unsigned long long* ctr, long long ntiles) {
+  const unsigned long long t = atomicAdd(ctr, 1ull);
+  if (t == (unsigned long long)ntiles + gridDim.x - 1) *ctr = 0ull;
+  return t;
+}
+__device__ __forceinline__ long long tile_first(unsigned long long* ctr, long long* s, long long ntiles) {
   if (!ctr) return blockIdx.x;
-  if (threadIdx.x == 0) *s = (long long)atomicAdd(ctr, 1ull);
+  if (threadIdx.x == 0) *s = (long long)tile_take(ctr, ntiles);
   __syncthreads();
   return *s;
 }
-__device__ __forceinline__ unsigned long long tile_prefetch(unsigned long long* ctr) {
-  return (ctr && threadIdx.x == 0) ? atomicAdd(ctr, 1ull) : 0ull;
+__device__ __forceinline__ unsigned long long tile_prefetch(unsigned long long* ctr, long long ntiles) {
+  return (ctr && threadIdx.x == 0) ? tile_take(ctr, ntiles) : 0ull;
 }
 __device__ __forceinline__ long long tile_next(unsigned long long* ctr, long long* s, long long tile,
                                                unsigned long long nxt) {
@@ -640,17 +648,19 @@ template <int L, class Ld>
 __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_NOISE)
     kp2_noise(const float4* __restrict__ twg, long long ntiles, int tpo, int Lout, Ld ld, P2ArrStore st,
               unsigned long long* ctr) {
+  chain_start();
   __shared__ long long s_tile;
   using G = P2Geom<L>;
   extern __shared__ __align__(16) float4 p2_smem[];
   float4* buf = p2_smem;
   float4* tw = p2_smem + G::Q * G::PLQ;
   p2_copy_table(tw, twg, G::NTW);
+  chain_wait();
   __syncthreads();
   const int q = threadIdx.x % G::Q, u = threadIdx.x / G::Q;
   unsigned bad = 0;
-  for (long long tile = tile_first(ctr, &s_tile); tile < ntiles;) {
-    const unsigned long long nxt = tile_prefetch(ctr);
+  for (long long tile = tile_first(ctr, &s_tile, ntiles); tile < ntiles;) {
+    const unsigned long long nxt = tile_prefetch(ctr, ntiles);
     const int o = (int)(tile / tpo);
     const int p = (int)(tile - (long long)o * tpo) * G::NP + 2 * q;
     P2 v[8];
@@ -732,6 +742,7 @@ template <int M, class Ld>
 __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_NOISE)
     kp2_noise3(const float4* __restrict__ twg, long long ntiles, int tpo, int Lout, Ld ld, P2ArrStore st,
                unsigned long long* ctr) {
+  chain_start();
   __shared__ long long s_tile;
   using G = P2Geom<M>;
   using G3 = P2Geom3<M>;
@@ -741,14 +752,15 @@ __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_NOISE)
   float4* tw = p2_smem + G::Q * G::PLQ;
   const float4* tw3 = tw + G::NTW;  // exp(+2 pi i n1 k2 / L) at (k2 - 1) M + n1, k2 = 1, 2
   p2_copy_table(tw, twg, G::NTW + 2 * M);
+  chain_wait();
   __syncthreads();
   const int tid = threadIdx.x;
   const int q = tid % G3::QS, u = tid / G3::QS;  // transform: sub-pencil slot, column
   const int pq = q / 3;
   const int gp = tid / (3 * G::TP), gi = tid - gp * (3 * G::TP);  // generation: pair, index
   unsigned bad = 0;
-  for (long long tile = tile_first(ctr, &s_tile); tile < ntiles;) {
-    const unsigned long long nxt = tile_prefetch(ctr);
+  for (long long tile = tile_first(ctr, &s_tile, ntiles); tile < ntiles;) {
+    const unsigned long long nxt = tile_prefetch(ctr, ntiles);
     const int o = (int)(tile / tpo);
     const int p0 = (int)(tile - (long long)o * tpo) * (2 * G3::PP);
     {  // noise x[n] of pair gp, elements j and j + L/2 per call
@@ -792,6 +804,7 @@ template <int M, int S>
 __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2C)
     kp2_c2c3(const float4* __restrict__ twg, long long ntiles, int tpo, int Lout, P2ArrLoad ld, P2ArrStore st,
              unsigned long long* ctr) {
+  chain_start();
   __shared__ long long s_tile;
   using G = P2Geom<M>;
   using G3 = P2Geom3<M>;
@@ -800,13 +813,14 @@ __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2C)
   float4* tw = p2_smem + G::Q * G::PLQ;
   const float4* tw3 = tw + G::NTW;
   p2_copy_table(tw, twg, G::NTW + 2 * M);
+  chain_wait();
   __syncthreads();
   const int tid = threadIdx.x;
   const int q = tid % G3::QS, u = tid / G3::QS;
   const int pq = q / 3, k2 = q - 3 * (q / 3);
   unsigned bad = 0;
-  for (long long tile = tile_first(ctr, &s_tile); tile < ntiles;) {
-    const unsigned long long nxt = tile_prefetch(ctr);
+  for (long long tile = tile_first(ctr, &s_tile, ntiles); tile < ntiles;) {
+    const unsigned long long nxt = tile_prefetch(ctr, ntiles);
     const int o = (int)(tile / tpo);
     const int p0 = (int)(tile - (long long)o * tpo) * (2 * G3::PP);
     // the three inputs of each radix-3 butterfly straight from global memory (the three
@@ -836,17 +850,19 @@ template <int L, int S>
 __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2C)
     kp2_c2c(const float4* __restrict__ twg, long long ntiles, int tpo, int Lout, P2ArrLoad ld, P2ArrStore st,
             unsigned long long* ctr) {
+  chain_start();
   __shared__ long long s_tile;
   using G = P2Geom<L>;
   extern __shared__ __align__(16) float4 p2_smem[];
   float4* buf = p2_smem;
   float4* tw = p2_smem + G::Q * G::PLQ;
   p2_copy_table(tw, twg, G::NTW);
+  chain_wait();
   __syncthreads();
   const int q = threadIdx.x % G::Q, u = threadIdx.x / G::Q;
   unsigned bad = 0;
-  for (long long tile = tile_first(ctr, &s_tile); tile < ntiles;) {
-    const unsigned long long nxt = tile_prefetch(ctr);
+  for (long long tile = tile_first(ctr, &s_tile, ntiles); tile < ntiles;) {
+    const unsigned long long nxt = tile_prefetch(ctr, ntiles);
     const int o = (int)(tile / tpo);
     const int p = (int)(tile - (long long)o * tpo) * G::NP + 2 * q;
     P2 v[8];
@@ -920,6 +936,7 @@ template <int L, int S>
 __global__ void __launch_bounds__(kP2Threads, 2)
     kp2_c2c_tma(const __grid_constant__ CUtensorMap src, const float4* __restrict__ twg, long long ntiles, int tpo,
                 int rows_per_outer, int Lin, int Lout, P2ArrStore st) {
+  chain_start();
   using G = P2Geom<L>;
   using M = P2Tma<L>;
   extern __shared__ __align__(128) float4 p2_tma_smem[];
@@ -935,6 +952,7 @@ __global__ void __launch_bounds__(kP2Threads, 2)
     mbar_fence_init();
   }
   p2_copy_table(tw, twg, G::NTW);
+  chain_wait();
   __syncthreads();
   const int q = tid % G::Q, u = tid / G::Q;
   unsigned bad = 0;
@@ -993,6 +1011,7 @@ template <int L, class Mid>
 __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_MID)
     kp2_c2c_mid(const float4* __restrict__ twf, const float4* __restrict__ twb, long long ntiles, int tpo,
                 int Lout, P2ArrLoad ld, Mid mid, P2ArrStore st, unsigned long long* ctr) {
+  chain_start();
   __shared__ long long s_tile;
   using G = P2Geom<L>;
   extern __shared__ __align__(16) float4 p2_smem[];
@@ -1001,11 +1020,12 @@ __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_MID)
   float4* tb = tf + G::NTW;
   p2_copy_table(tf, twf, G::NTW);
   p2_copy_table(tb, twb, G::NTW);
+  chain_wait();
   __syncthreads();
   const int q = threadIdx.x % G::Q, u = threadIdx.x / G::Q;
   unsigned bad = 0;
-  for (long long tile = tile_first(ctr, &s_tile); tile < ntiles;) {
-    const unsigned long long nxt = tile_prefetch(ctr);
+  for (long long tile = tile_first(ctr, &s_tile, ntiles); tile < ntiles;) {
+    const unsigned long long nxt = tile_prefetch(ctr, ntiles);
     const int o = (int)(tile / tpo);
     const int p = (int)(tile - (long long)o * tpo) * G::NP + 2 * q;
     P2 v[8];
@@ -1043,12 +1063,14 @@ __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_MID)
 template <int L, class St>
 __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2R)
     kp2_c2r(const float4* __restrict__ twg, long long ntiles, int Lout, P2RowLoad ld, St st) {
+  chain_start();
   using G = P2Geom<L>;
   extern __shared__ __align__(16) float4 p2_smem[];
   float4* buf = p2_smem;
   float4* tw = p2_smem + G::Q * G::PLQ;
   const float4* twT = tw + G::NTW;  // exp(+2 pi i m / 2L), m < L
   p2_copy_table(tw, twg, G::NTW + L);
+  chain_wait();
   __syncthreads();
   const int u = threadIdx.x % G::TP, q = threadIdx.x / G::TP;
   unsigned bad = 0;
@@ -1124,6 +1146,7 @@ struct P2Bulk {
 template <int L, class St>
 __global__ void __launch_bounds__(kP2Threads, 2)
     kp2_c2r_bulk(const float4* __restrict__ twg, long long ntiles, int Lout, P2RowLoad ld, St st) {
+  chain_start();
   using G = P2Geom<L>;
   extern __shared__ __align__(128) float4 p2_bulk_smem[];
   const unsigned rs = ld.rowstride;
@@ -1141,6 +1164,7 @@ __global__ void __launch_bounds__(kP2Threads, 2)
     mbar_fence_init();
   }
   p2_copy_table(tw, twg, G::NTW + L);
+  chain_wait();
   __syncthreads();
   const int u = tid % G::TP, q = tid / G::TP;
   unsigned bad = 0;
@@ -1214,6 +1238,7 @@ __global__ void __launch_bounds__(kP2Threads, 2)
 template <int M, class St>
 __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2R)
     kp2_c2r3(const float4* __restrict__ twg, long long ntiles, int Lout, P2RowLoad ld, St st) {
+  chain_start();
   using G = P2Geom<M>;
   using G3 = P2Geom3<M>;
   constexpr int L = G3::L;
@@ -1223,6 +1248,7 @@ __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2R)
   const float4* tw3 = tw + G::NTW;          // radix-3 twiddles, 2M entries
   const float4* twT = tw3 + 2 * M;          // exp(+2 pi i m / 2L), m < L
   p2_copy_table(tw, twg, G::NTW + 2 * M + L);
+  chain_wait();
   __syncthreads();
   const int tid = threadIdx.x;
   const int q = tid % G3::QS, u = tid / G3::QS;
@@ -1427,12 +1453,14 @@ struct P2RowStore {
 template <int L, class Ld>
 __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2R)
     kp2_r2c(const float4* __restrict__ twg, long long ntiles, Ld ld, P2RowStore st) {
+  chain_start();
   using G = P2Geom<L>;
   extern __shared__ __align__(16) float4 p2_smem[];
   float4* buf = p2_smem;
   float4* tw = p2_smem + G::Q * G::PLQ;
   const float4* twT = tw + G::NTW;  // exp(+2 pi i m / 2L), m < L
   p2_copy_table(tw, twg, G::NTW + L);
+  chain_wait();
   __syncthreads();
   const int u = threadIdx.x % G::TP, q = threadIdx.x / G::TP;
   unsigned bad = 0;
