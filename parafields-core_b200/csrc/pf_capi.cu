@@ -913,7 +913,7 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
     P->grid_cap = P->tune_grid[2];
     const size_t left = (size_t)(g.domain - (size_t)(dst - out));
     if constexpr (F32) {
-      if (P->tune_variant[2] != 1 && g.T[0] % 2 == 0 && (p2_length(g.T[0] / 2) || p2_length3(g.T[0] / 2))) {
+      if (P->tune_variant[2] == 2 && g.T[0] % 2 == 0 && p2_length(g.T[0] / 2)) {  // rows staged by bulk copies
         P2RowLoad rl;
         rl.ptr = (const float2*)src;
         rl.rowstride = (unsigned)P0;
@@ -929,9 +929,8 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
         ps.np = (int)nrows;
         ps.Lout = g.n[0];
         ps.vec = (g.n[0] % 2 == 0 && ((uintptr_t)dst & 7u) == 0) ? 1 : 0;
-        if (P->tune_variant[2] == 2 && p2_bulk_ok(rl, g.T[0] / 2))  // rows staged by bulk copies
+        if (p2_bulk_ok(rl, g.T[0] / 2))
           return p2_c2r_bulk(P, "gen_c2r_d0_bulk", g.T[0] / 2, g.n[0], nrows, rl, ps, b3);
-        return p2_c2r(P, "gen_c2r_d0", g.T[0] / 2, g.n[0], nrows, rl, ps, b3);
       }
     }
     FieldRowStore<S> fr{dst, g.n[0], transform, P->desc.boxcox_lambda, (unsigned)left,
@@ -954,12 +953,12 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
     void* src = (char*)W1 + sizeof(cx<T>) * (size_t)w1_plane * z0;
     const double b2 = (double)T0c * nz * (g.T[1] + g.n[1]) * e;
     P->grid_cap = P->tune_grid[1];
-    const bool p2ok = F32 && (p2_length(g.T[1]) || p2_length3(g.T[1])) && p2_view_ok(src, P0, w1_plane, nz) &&
+    const bool p2ok = F32 && p2_length(g.T[1]) && p2_view_ok(src, P0, w1_plane, nz) &&
                       p2_view_ok(W2, P0, w2_plane, nz);
     const P2ArrLoad l1 = p2_load(P, src, P0, w1_plane, g.T[1], T0c);
-    if (p2ok && P->tune_variant[1] == 2 && p2_length(g.T[1]) && p2_tma_ok(P, l1, nz))  // tiles staged by TMA
+    if (p2ok && P->tune_variant[1] == 2 && p2_tma_ok(P, l1, nz))  // tiles staged by TMA
       TRY(p2_c2c_tma<+1>(P, "gen_c2c_d1_tma", g.T[1], g.n[1], T0c, nz, l1, p2_store(P, W2, P0, w2_plane, T0c), b2));
-    else if (p2ok && P->tune_variant[1] != 1)
+    else if (p2ok && P->tune_variant[1] != 1 && p2_strided(g.T[1]))
       TRY(p2_c2c<+1>(P, "gen_c2c_d1", g.T[1], g.n[1], T0c, nz, l1, p2_store(P, W2, P0, w2_plane, T0c), b2));
     else
       TRY((run_pass<T, false, +1>(P, "gen_c2c_d1", g.T[1], g.n[1], T0c, nz,
@@ -1165,19 +1164,6 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
       }
       return fail(PF_ERR_STATE, "internal error: fused dot product on a matvec without paired rows");
     }
-    if constexpr (std::is_same<T, float>::value) {
-      if (p2rows) {
-        P2RowLoad rl;
-        rl.ptr = (const float2*)X;
-        rl.rowstride = (unsigned)P0;
-        rl.n = (unsigned)std::min<size_t>(cap_of(P, X) / sizeof(float2), 0xffffffffu);
-        rl.Lin = T0c;
-        rl.np = (int)nrows;
-        P2FieldStoreT<S> ps{out, g.n[0], 0, 0.f, (unsigned)g.domain, (int)nrows, g.n[0],
-                            pair_ok && ((uintptr_t)out % (2 * sizeof(S))) == 0 ? 1 : 0};
-        return p2_c2r(P, "mv_c2r_d0", g.T[0] / 2, g.n[0], nrows, rl, ps, b);
-      }
-    }
     return run_real_pass<T, false>(P, "mv_c2r_d0", g.T[0], g.n[0], nrows, arr_load<cx<T>>(P, X, 1, 0, P0, T0c), fs, b);
   };
   if (g.dim == 2) {
@@ -1185,13 +1171,8 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
     TRY(workspace(P, 2, sizeof(cx<T>) * (size_t)P0 * g.n[1], &X1));
     TRY(fwd_rows(X1, g.n[1]));
     const double bf1 = (double)T0c * (2.0 * g.n[1] * e + g.T[1] * lb);
-    if (std::is_same<T, float>::value && p2_length(g.T[1]) && p2_view_ok(X1, P0, 0, 1))
-      TRY(p2_c2c_mid(P, "mv_fused_d1", g.T[1], g.n[1], T0c, 1, p2_load(P, X1, P0, 0, g.n[1], T0c), mid,
-                     p2_store(P, X1, P0, 0, T0c), bf1));
-    else
-      TRY((run_pass<T, false, -1>(P, "mv_fused_d1", g.T[1], g.n[1], T0c, 1,
-                                              arr_load<cx<T>>(P, X1, P0, 0, 1, g.n[1]), mid,
-                                              arr_store<cx<T>>(P, X1, P0, 0, 1), bf1)));
+    TRY((run_pass<T, false, -1>(P, "mv_fused_d1", g.T[1], g.n[1], T0c, 1, arr_load<cx<T>>(P, X1, P0, 0, 1, g.n[1]), mid,
+                                arr_store<cx<T>>(P, X1, P0, 0, 1), bf1)));
     return inv_rows(X1, g.n[1]);
   }
   void *X1 = nullptr, *X2 = nullptr;
@@ -1203,7 +1184,7 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
   // the strided passes along dim 1 take the paired kernels where the torus length and the
   // views allow (FP32 transforms), as in generation
   const long long w1o = (long long)P0 * g.n[1];
-  const bool p2d1 = std::is_same<T, float>::value && p2_length(g.T[1]) && p2_view_ok(X1, P0, w1o, g.n[2]) &&
+  const bool p2d1 = std::is_same<T, float>::value && p2_strided(g.T[1]) && p2_view_ok(X1, P0, w1o, g.n[2]) &&
                     p2_view_ok(X2, P0, s2, g.n[2]);
   const double bd1 = (double)T0c * g.n[2] * (g.n[1] + g.T[1]) * e;
   if (p2d1)
@@ -1215,13 +1196,8 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
                                             arr_store<cx<T>>(P, X2, P0, s2, 1), bd1)));
   // forward along dim 2, eigenvalue factor, backward along dim 2 (pencils k0 x k1)
   const double bf2 = (double)T0c * g.T[1] * (2.0 * g.n[2] * e + g.T[2] * lb);
-  if (std::is_same<T, float>::value && p2_length(g.T[2]) && p2_view_ok(X2, s2, P0, g.T[1]))
-    TRY(p2_c2c_mid(P, "mv_fused_d2", g.T[2], g.n[2], T0c, g.T[1], p2_load(P, X2, s2, P0, g.n[2], T0c), mid,
-                   p2_store(P, X2, s2, P0, T0c), bf2));
-  else
-    TRY((run_pass<T, false, -1>(P, "mv_fused_d2", g.T[2], g.n[2], T0c, g.T[1],
-                                            arr_load<cx<T>>(P, X2, s2, P0, 1, g.n[2]), mid,
-                                            arr_store<cx<T>>(P, X2, s2, P0, 1), bf2)));
+  TRY((run_pass<T, false, -1>(P, "mv_fused_d2", g.T[2], g.n[2], T0c, g.T[1],
+                              arr_load<cx<T>>(P, X2, s2, P0, 1, g.n[2]), mid, arr_store<cx<T>>(P, X2, s2, P0, 1), bf2)));
   if (p2d1)
     TRY(p2_c2c<+1>(P, "mv_c2c_d1i", g.T[1], g.n[1], T0c, g.n[2], p2_load(P, X2, P0, s2, g.T[1], T0c),
                    p2_store(P, X1, P0, w1o, T0c), bd1));

@@ -33,8 +33,7 @@ constexpr int pick_radix(int m) { return m % 8 == 0 ? 8 : (m % 4 == 0 ? 4 : 2); 
 // and in the two-stream batch its CTAs fit beside the other stream's kernels (256^3
 // Matern-3/2 batch: 0.388 against 0.401 ms per realization).  At 64 registers the
 // complex-to-real pass spills and runs slower alone (0.088 against 0.077 ms) and in the
-// batch, so it keeps 3.  The fused matvec pass spills a few words at 64 registers but waits
-// on its gathers, and the extra warps win (128^3 C^-1: 0.066 against 0.075 ms).
+// batch, so it keeps 3.
 #ifndef PF_P2_MIN_NOISE
 #define PF_P2_MIN_NOISE 4
 #endif
@@ -43,9 +42,6 @@ constexpr int pick_radix(int m) { return m % 8 == 0 ? 8 : (m % 4 == 0 ? 4 : 2); 
 #endif
 #ifndef PF_P2_MIN_C2R
 #define PF_P2_MIN_C2R 3
-#endif
-#ifndef PF_P2_MIN_MID
-#define PF_P2_MIN_MID 4
 #endif
 
 struct P2 {
@@ -163,9 +159,10 @@ __device__ __forceinline__ int p2_slot(int PLQ, int q, int j) { return q * PLQ +
 
 // stages 2.. of the transform: v holds the thread's 8 values of stage Ns's input
 // (after stage 1 they are in buf).  Out(j, P2) receives the final outputs.
+// (threads with act = false only take part in the barriers)
 template <int L, int S, int Ns, int TWOFF, class Out>
 __device__ __forceinline__ void p2_stages(P2 (&v)[8], float4* buf, const float4* tw, int u, int q,
-                                          const Out& out) {
+                                          const Out& out, bool act = true) {
   using G = P2Geom<L>;
   constexpr int R = pick_radix(L / Ns);
   constexpr int NB = 8 / R;
@@ -176,12 +173,14 @@ __device__ __forceinline__ void p2_stages(P2 (&v)[8], float4* buf, const float4*
   // per thread, the rest compile-time offsets
   static_assert(G::TP % 8 == 0 && NBF % 8 == 0 && Ns % 8 == 0, "slot offsets need multiples of 8");
   const float4* rd = buf + p2_slot(G::PLQ, q, u);
+  if (act)
 #pragma unroll
-  for (int i = 0; i < NB; i++) {
+    for (int i = 0; i < NB; i++) {
 #pragma unroll
-    for (int r = 0; r < R; r++) v[i * R + r] = p2_of(rd[(i * G::TP + r * NBF) / 8 * 9]);
-  }
+      for (int r = 0; r < R; r++) v[i * R + r] = p2_of(rd[(i * G::TP + r * NBF) / 8 * 9]);
+    }
   __syncthreads();
+  if (act)
 #pragma unroll
   for (int i = 0; i < NB; i++) {
     const int t = u + i * G::TP;
@@ -198,19 +197,21 @@ __device__ __forceinline__ void p2_stages(P2 (&v)[8], float4* buf, const float4*
       for (int r = 0; r < R; r++) wr[r * Ns / 8 * 9] = slot_of(v[i * R + r]);
     }
   }
-  if constexpr (!LAST) p2_stages<L, S, Ns * R, TWOFF + (R - 1) * Ns>(v, buf, tw, u, q, out);
+  if constexpr (!LAST) p2_stages<L, S, Ns * R, TWOFF + (R - 1) * Ns>(v, buf, tw, u, q, out, act);
 }
 
 // whole transform from the stage-1 inputs v[r] = element u + r*L/8
 template <int L, int S, class Out>
 __device__ __forceinline__ void p2_transform(P2 (&v)[8], float4* buf, const float4* tw, int u, int q,
-                                             const Out& out) {
+                                             const Out& out, bool act = true) {
   using G = P2Geom<L>;
-  pdft8<S>(v);
-  float4* wr = buf + p2_slot(G::PLQ, q, u * 8);  // u*8 + r stays within one group of 8
+  if (act) {
+    pdft8<S>(v);
+    float4* wr = buf + p2_slot(G::PLQ, q, u * 8);  // u*8 + r stays within one group of 8
 #pragma unroll
-  for (int r = 0; r < 8; r++) wr[r] = slot_of(v[r]);
-  p2_stages<L, S, 8, 0>(v, buf, tw, u, q, out);
+    for (int r = 0; r < 8; r++) wr[r] = slot_of(v[r]);
+  }
+  p2_stages<L, S, 8, 0>(v, buf, tw, u, q, out, act);
 }
 
 __device__ __forceinline__ void p2_copy_table(float4* dst, const float4* __restrict__ src, int n) {
@@ -686,60 +687,39 @@ __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_NOISE)
 // length-L backward transform split as
 //   X[3 k1 + k2] = sum_n1 W_M^(n1 k1) [ W_L^(n1 k2) sum_n2 x[n1 + M n2] W_3^(n2 k2) ],
 // i.e. a radix-3 step with twiddles, then three paired M-point transforms per pencil
-// pair (one per k2).  A tile holds PP pencil pairs: their noise is first generated into
-// shared memory (the exchange buffer, PP L slots), then every thread reads the three inputs
-// of its radix-3 butterflies, and thread slot q transforms sub-pencil k2 = q % 3 of pair
-// q / 3.  The block has exactly 3 PP M/8 threads.
+// pair (one per k2).  A tile holds PP = 512 / M pencil pairs.  A thread generates the six
+// elements of its pair's butterflies n1 and n1 + M/2 (three generator calls: n1, n1 + M and
+// n1 + M/2 with their partners half a length further) and runs both radix-3 steps in
+// registers; the 3 PP sub-pencils pass through shared memory once, then 3 M/8 threads per pair
+// transform them.  Adjacent threads hold adjacent pairs, so eigenvalue loads cover 8 PP bytes.
+// Staging the noise first and letting each thread compute one of a butterfly's three outputs
+// from three shared-memory reads took 280 us for 384 points of 384 x 193 pencils; this takes 229 at
+// 4 resident CTAs per SM (64 registers, some spilled) and 217 at 3.
 // ---------------------------------------------------------------------------
 template <int M>
 struct P2Geom3 {
   using G = P2Geom<M>;
   static constexpr int L = 3 * M;
-  static constexpr int PP = kP2Threads / (3 * G::TP);  // pencil pairs per tile
-  static constexpr int NT = PP * 3 * G::TP;            // threads per CTA
-  static constexpr int QS = 3 * PP;                    // sub-pencil slots
-  static_assert(PP >= 1 && QS <= G::Q, "sub-pencil slots fit the exchange buffer");
-  static_assert(PP * L <= G::Q * G::PLQ, "the tile's noise fits the exchange buffer");
+  static constexpr int PP = 512 / M;    // pencil pairs per tile: 256 threads of M/2 per pair
+  static constexpr int QS = 3 * PP;     // sub-pencils
+  static_assert(PP * (M / 2) == kP2Threads && QS * G::TP <= kP2Threads && QS <= G::Q, "tile geometry");
 };
 
-// Radix-3 step and M-point transforms of a tile staged in the exchange buffer (pair g's
-// element n at buf[g L + n]): thread slot q transforms sub-pencil k2 = q % 3 of pair q / 3;
-// Out(j, value) receives output j = 3 k1 + k2.  Sign S of the transform (W = exp(S 2 pi i / .)).
-// output k2 of the radix-3 butterfly of (a, b, c) (elements n1, n1 + M, n1 + 2M), times the
-// twiddle w = W_L^(n1 k2) (unused for k2 = 0)
-template <int S>
-__device__ __forceinline__ P2 p2_radix3_point(const P2& a, const P2& b, const P2& c, int k2, float4 w) {
-  const P2 sm = padd(b, c);
-  if (k2 == 0) return padd(a, sm);
-  // W_3^(k2) = -1/2 + i S sin(2 pi k2 / 3): + sqrt(3)/2 for (S, k2) = (+, 1) and (-, 2)
-  const float sq3 = (k2 == 1) == (S > 0) ? 0.86602540378443865f : -0.86602540378443865f;
-  const float2 hf = make_float2(-0.5f, -0.5f), s3 = make_float2(sq3, sq3), ns3 = make_float2(-sq3, -sq3);
-  const P2 df = psub(b, c);
-  // a - (b + c) / 2 + i s3 (b - c)
-  const P2 y = {f2fma(hf, sm.re, f2fma(ns3, df.im, a.re)), f2fma(hf, sm.im, f2fma(s3, df.re, a.im))};
-  return ptw(y, w);
-}
-
-template <int M, int S, class Out>
-__device__ __forceinline__ void p2_radix3_transform(float4* buf, const float4* tw, const float4* tw3, int u, int q,
-                                                    const Out& out) {
-  using G = P2Geom<M>;
-  constexpr int L = 3 * M;
-  const int pq = q / 3, k2 = q - 3 * (q / 3);
-  P2 v[8];
-  const float4* xs = buf + pq * L;
-#pragma unroll
-  for (int r = 0; r < 8; r++) {
-    const int n1 = u + r * G::TP;
-    v[r] = p2_radix3_point<S>(p2_of(xs[n1]), p2_of(xs[n1 + M]), p2_of(xs[n1 + 2 * M]), k2,
-                              k2 ? tw3[(k2 - 1) * M + n1] : make_float4(1.f, 1.f, 0.f, 0.f));
-  }
-  __syncthreads();  // every thread has read the staged tile before the transform writes the buffer
-  p2_transform<M, S>(v, buf, tw, u, q, [&](int k1, const P2& x) { out(3 * k1 + k2, x); });
+// backward radix-3 step of (a, b, c) (elements n1, n1 + M, n1 + 2M): outputs k2 = 0, 1, 2, the last
+// two times their twiddles w1 = W_L^n1, w2 = W_L^(2 n1)
+__device__ __forceinline__ void p2_radix3(P2& a, P2& b, P2& c, float4 w1, float4 w2) {
+  const P2 s = padd(b, c), d = psub(b, c);
+  const float2 hf = make_float2(-0.5f, -0.5f), k = make_float2(0.86602540378443865f, 0.86602540378443865f),
+               nk = make_float2(-0.86602540378443865f, -0.86602540378443865f);
+  const P2 m = {f2fma(hf, s.re, a.re), f2fma(hf, s.im, a.im)};
+  a = padd(a, s);
+  // m + i k d and m - i k d
+  b = ptw(P2{f2fma(nk, d.im, m.re), f2fma(k, d.re, m.im)}, w1);
+  c = ptw(P2{f2fma(k, d.im, m.re), f2fma(nk, d.re, m.im)}, w2);
 }
 
 template <int M, class Ld>
-__global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_NOISE)
+__global__ void __launch_bounds__(kP2Threads, 3)
     kp2_noise3(const float4* __restrict__ twg, long long ntiles, int tpo, int Lout, Ld ld, P2ArrStore st,
                unsigned long long* ctr) {
   chain_start();
@@ -748,96 +728,56 @@ __global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_NOISE)
   using G3 = P2Geom3<M>;
   constexpr int L = G3::L;
   extern __shared__ __align__(16) float4 p2_smem[];
-  float4* buf = p2_smem;  // exchange buffer; also the tile's noise, pair g at buf[g L + n]
+  float4* buf = p2_smem;  // exchange buffer; sub-pencil 3 pair + k2
   float4* tw = p2_smem + G::Q * G::PLQ;
   const float4* tw3 = tw + G::NTW;  // exp(+2 pi i n1 k2 / L) at (k2 - 1) M + n1, k2 = 1, 2
   p2_copy_table(tw, twg, G::NTW + 2 * M);
   chain_wait();
   __syncthreads();
   const int tid = threadIdx.x;
-  const int q = tid % G3::QS, u = tid / G3::QS;  // transform: sub-pencil slot, column
-  const int pq = q / 3;
-  const int gp = tid / (3 * G::TP), gi = tid - gp * (3 * G::TP);  // generation: pair, index
-  unsigned bad = 0;
-  for (long long tile = tile_first(ctr, &s_tile, ntiles); tile < ntiles;) {
-    const unsigned long long nxt = tile_prefetch(ctr, ntiles);
-    const int o = (int)(tile / tpo);
-    const int p0 = (int)(tile - (long long)o * tpo) * (2 * G3::PP);
-    {  // noise x[n] of pair gp, elements j and j + L/2 per call
-      const int p = p0 + 2 * gp;
-      float4* xs = buf + gp * L;
-      if (ld.noise) {
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-          const int j = gi + r * (3 * G::TP);
-          P2 x0, x1;
-          ld.template load2<L>(p, j, o, x0, x1, bad);
-          xs[j] = slot_of(x0);
-          xs[j + L / 2] = slot_of(x1);
-        }
-      } else {
-        const auto t = ld.template tile<L>(p, o, bad);
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-          const int j = gi + r * (3 * G::TP);
-          P2 x0, x1;
-          ld.template load2t<L>(t, j, x0, x1);
-          xs[j] = slot_of(x0);
-          xs[j + L / 2] = slot_of(x1);
-        }
-      }
-    }
-    __syncthreads();
-    const P2ArrStore::Tile so = st.tile(p0 + 2 * pq, o, Lout, bad);
-    p2_radix3_transform<M, +1>(buf, tw, tw3, u, q, [&](int j, const P2& x) {
-      if (j < Lout) st.store_t(so, j, x);
-    });
-    tile = tile_next(ctr, &s_tile, tile, nxt);
-  }
-  p2_report(bad);
-}
-
-// Strided complex pass of length L = 3 M (pencils p, p+1 adjacent): every thread loads the
-// three inputs of its radix-3 butterflies itself, then the paired M-point transforms run as
-// in kp2_noise3.
-template <int M, int S>
-__global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2C)
-    kp2_c2c3(const float4* __restrict__ twg, long long ntiles, int tpo, int Lout, P2ArrLoad ld, P2ArrStore st,
-             unsigned long long* ctr) {
-  chain_start();
-  __shared__ long long s_tile;
-  using G = P2Geom<M>;
-  using G3 = P2Geom3<M>;
-  extern __shared__ __align__(16) float4 p2_smem[];
-  float4* buf = p2_smem;
-  float4* tw = p2_smem + G::Q * G::PLQ;
-  const float4* tw3 = tw + G::NTW;
-  p2_copy_table(tw, twg, G::NTW + 2 * M);
-  chain_wait();
-  __syncthreads();
-  const int tid = threadIdx.x;
-  const int q = tid % G3::QS, u = tid / G3::QS;
+  const int gp = tid % G3::PP, n1 = tid / G3::PP;    // generation: pair, butterflies n1 and n1 + M/2
+  const bool act = tid < G3::QS * G::TP;             // transform: sub-pencil, column
+  const int q = tid % G3::QS, u = act ? tid / G3::QS : 0;
   const int pq = q / 3, k2 = q - 3 * (q / 3);
   unsigned bad = 0;
   for (long long tile = tile_first(ctr, &s_tile, ntiles); tile < ntiles;) {
     const unsigned long long nxt = tile_prefetch(ctr, ntiles);
     const int o = (int)(tile / tpo);
     const int p0 = (int)(tile - (long long)o * tpo) * (2 * G3::PP);
-    // the three inputs of each radix-3 butterfly straight from global memory (the three
-    // threads of a pencil pair that share them read the same addresses, served by L1)
-    const P2ArrLoad::Tile lt = ld.tile(p0 + 2 * pq, o, bad);
-    P2 v[8];
+    P2 x[6];  // elements n1 + r M/2
+    {
+      const int p = p0 + 2 * gp;
+      if (ld.noise) {
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int n1 = u + r * G::TP;
-      v[r] = p2_radix3_point<S>(ld.load_t(lt, n1), ld.load_t(lt, n1 + M), ld.load_t(lt, n1 + 2 * M), k2,
-                                k2 ? tw3[(k2 - 1) * M + n1] : make_float4(1.f, 1.f, 0.f, 0.f));
+        for (int r = 0; r < 3; r++) ld.template load2<L>(p, n1 + r * (M / 2), o, x[r], x[r + 3], bad);
+      } else {
+        const auto t = ld.template tile<L>(p, o, bad);
+#pragma unroll
+        for (int r = 0; r < 3; r++) ld.template load2t<L>(t, n1 + r * (M / 2), x[r], x[r + 3]);
+      }
     }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int m = n1 + h * (M / 2);
+      p2_radix3(x[h], x[h + 2], x[h + 4], tw3[m], tw3[M + m]);
+      float4* const w = buf + p2_slot(G::PLQ, 3 * gp, m);
+      w[0] = slot_of(x[h]);
+      w[G::PLQ] = slot_of(x[h + 2]);
+      w[2 * G::PLQ] = slot_of(x[h + 4]);
+    }
+    __syncthreads();
+    P2 v[8];
+    if (act) {
+      const float4* const rd = buf + p2_slot(G::PLQ, q, u);
+#pragma unroll
+      for (int r = 0; r < 8; r++) v[r] = p2_of(rd[r * G::TP / 8 * 9]);
+    }
+    __syncthreads();  // the sub-pencils are read before the transform writes the buffer
     const P2ArrStore::Tile so = st.tile(p0 + 2 * pq, o, Lout, bad);
-    p2_transform<M, S>(v, buf, tw, u, q, [&](int k1, const P2& x) {
+    p2_transform<M, +1>(v, buf, tw, u, q, [&](int k1, const P2& y) {
       const int j = 3 * k1 + k2;
-      if (j < Lout) st.store_t(so, j, x);
-    });
+      if (j < Lout) st.store_t(so, j, y);
+    }, act);
     tile = tile_next(ctr, &s_tile, tile, nxt);
   }
   p2_report(bad);
@@ -999,59 +939,6 @@ __global__ void __launch_bounds__(kP2Threads, 2)
   }
   if ((bad & 2u) && tid == 0 && pending_next)  // a copy issued before the failed wait: bounded wait for it
     mbar_wait_bounded(&bar[(k & 1) ^ 1], (uint32_t)((k + 1) >> 1) & 1u);
-  p2_report(bad);
-}
-
-// ---------------------------------------------------------------------------
-// Fused strided pass of the matvec: forward transform, a per-element operator (Mid, e.g.
-// the eigenvalue factor) and the backward transform of the same pencils, the spectrum
-// staying in shared memory between the two (tables of both directions in shared memory).
-// ---------------------------------------------------------------------------
-template <int L, class Mid>
-__global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_MID)
-    kp2_c2c_mid(const float4* __restrict__ twf, const float4* __restrict__ twb, long long ntiles, int tpo,
-                int Lout, P2ArrLoad ld, Mid mid, P2ArrStore st, unsigned long long* ctr) {
-  chain_start();
-  __shared__ long long s_tile;
-  using G = P2Geom<L>;
-  extern __shared__ __align__(16) float4 p2_smem[];
-  float4* buf = p2_smem;
-  float4* tf = p2_smem + G::Q * G::PLQ;
-  float4* tb = tf + G::NTW;
-  p2_copy_table(tf, twf, G::NTW);
-  p2_copy_table(tb, twb, G::NTW);
-  chain_wait();
-  __syncthreads();
-  const int q = threadIdx.x % G::Q, u = threadIdx.x / G::Q;
-  unsigned bad = 0;
-  for (long long tile = tile_first(ctr, &s_tile, ntiles); tile < ntiles;) {
-    const unsigned long long nxt = tile_prefetch(ctr, ntiles);
-    const int o = (int)(tile / tpo);
-    const int p = (int)(tile - (long long)o * tpo) * G::NP + 2 * q;
-    P2 v[8];
-    const P2ArrLoad::Tile lt = ld.tile(p, o, bad);
-#pragma unroll
-    for (int r = 0; r < 8; r++) v[r] = ld.load_t(lt, u + r * G::TP);
-    // forward transform; its outputs land in the exchange buffer (its last stage has read
-    // the buffer and passed a barrier before the first output is written)
-    p2_transform<L, -1>(v, buf, tf, u, q, [&](int j, const P2& x) { buf[p2_slot(G::PLQ, q, j)] = slot_of(x); });
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int j = u + r * G::TP;
-      const P2 x = p2_of(buf[p2_slot(G::PLQ, q, j)]);
-      cx<float> a = mk<float>(0.f, 0.f), b = a;  // pencils beyond the last one stay zero
-      if (p < ld.np) a = mid.template operator()<float>(p, j, o, mk<float>(x.re.x, x.im.x));
-      if (p + 1 < ld.np) b = mid.template operator()<float>(p + 1, j, o, mk<float>(x.re.y, x.im.y));
-      v[r] = {make_float2(a.x, b.x), make_float2(a.y, b.y)};
-    }
-    __syncthreads();
-    const P2ArrStore::Tile so = st.tile(p, o, Lout, bad);
-    p2_transform<L, +1>(v, buf, tb, u, q, [&](int j, const P2& x) {
-      if (j < Lout) st.store_t(so, j, x);
-    });
-    tile = tile_next(ctr, &s_tile, tile, nxt);
-  }
   p2_report(bad);
 }
 
@@ -1228,62 +1115,6 @@ __global__ void __launch_bounds__(kP2Threads, 2)
   }
   if ((bad & 2u) && tid == 0 && pending_next)  // a copy issued before the failed wait: bounded wait for it
     mbar_wait_bounded(&bar[(k & 1) ^ 1], (uint32_t)((k + 1) >> 1) & 1u);
-  p2_report(bad);
-}
-
-// Complex-to-real rows of length L = 3 M (2L reals from L+1 complex, FFTW c2r semantics as
-// kp2_c2r): the rows' pre-processed values Z[m] = (X[m] + conj X[L-m]) + i w^m (X[m] -
-// conj X[L-m]) of the tile's row pairs are staged in the exchange buffer, then the radix-3
-// step and the paired M-point transforms run as in kp2_noise3; output j holds reals 2j, 2j+1.
-template <int M, class St>
-__global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2R)
-    kp2_c2r3(const float4* __restrict__ twg, long long ntiles, int Lout, P2RowLoad ld, St st) {
-  chain_start();
-  using G = P2Geom<M>;
-  using G3 = P2Geom3<M>;
-  constexpr int L = G3::L;
-  extern __shared__ __align__(16) float4 p2_smem[];
-  float4* buf = p2_smem;
-  float4* tw = p2_smem + G::Q * G::PLQ;
-  const float4* tw3 = tw + G::NTW;          // radix-3 twiddles, 2M entries
-  const float4* twT = tw3 + 2 * M;          // exp(+2 pi i m / 2L), m < L
-  p2_copy_table(tw, twg, G::NTW + 2 * M + L);
-  chain_wait();
-  __syncthreads();
-  const int tid = threadIdx.x;
-  const int q = tid % G3::QS, u = tid / G3::QS;
-  const int pq = q / 3;
-  const int gp = tid / (3 * G::TP), gi = tid - gp * (3 * G::TP);
-  unsigned bad = 0;
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int p0 = (int)tile * (2 * G3::PP);
-    {
-      const int p = p0 + 2 * gp;
-      float4* zs = buf + gp * L;
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        const int m = gi + r * (3 * G::TP);
-        float2 xa = ld.one(p, m, bad), xb = ld.one(p + 1, m, bad);
-        float2 ya = ld.one(p, L - m, bad), yb = ld.one(p + 1, L - m, bad);
-        if (m == 0) {
-          xa.y = 0.f;
-          xb.y = 0.f;
-          ya.y = 0.f;
-          yb.y = 0.f;
-        }
-        const P2 X = p2_ab(xa, xb), Y = p2_ab(ya, yb);
-        const P2 sv = {f2add(X.re, Y.re), f2sub(X.im, Y.im)};
-        const P2 dv = {f2sub(X.re, Y.re), f2add(X.im, Y.im)};
-        const P2 t = ptw(dv, twT[m]);
-        zs[m] = slot_of(P2{f2sub(sv.re, t.im), f2add(sv.im, t.re)});
-      }
-    }
-    __syncthreads();
-    const int p = p0 + 2 * pq;
-    p2_radix3_transform<M, +1>(buf, tw, tw3, u, q, [&](int j, const P2& z) {
-      if (2 * j < Lout) st.store(p, j, z, bad);
-    });
-  }
   p2_report(bad);
 }
 
