@@ -198,6 +198,17 @@ struct ProfRec {
 
 struct pf_learned;
 
+// lengths, tile and launch geometry of one any-length pass; no caller's pointer is in it
+struct GPrep {
+  const void* kind;  // kernel instantiation
+  int L, Lout;
+  long long npencil, nouter;
+  int nt;
+  unsigned grid;
+  size_t smem;
+  alignas(16) unsigned char args[sizeof(GArgs<double>)];
+};
+
 struct pf_plan {
   pf_field_desc desc;
   Geom g;
@@ -278,6 +289,9 @@ struct pf_plan {
   // kernels may start while their predecessor in the stream drains (launch_chained); off while
   // two streams of a batch share the SMs, where waiting blocks would hold the other's places
   bool chain = true;
+  volatile unsigned* err_words = nullptr;  // the device's error words (error_words)
+  // geometry of the any-length passes this plan has launched (g_launch)
+  std::vector<GPrep> gprep;
 };
 
 static pf_status dalloc(pf_plan* P, void** p, size_t bytes) {
@@ -423,6 +437,35 @@ static pf_status set_smem(K kernel, size_t smem) {
   return PF_OK;
 }
 
+// what the runtime was told and answered about a kernel on a device: shared memory it may take,
+// resident blocks per SM at one block shape (both calls cost about as much as a launch)
+struct KernelFacts {
+  size_t smem = 0;
+  std::map<std::pair<int, size_t>, int> resident;
+};
+static std::mutex g_kernel_mu;
+static std::map<std::pair<const void*, int>, KernelFacts> g_kernels;
+
+// allows `smem` bytes for the kernel; per_sm (may be NULL) = resident blocks of `threads`
+template <typename K>
+static pf_status kernel_ready(pf_plan* P, K kern, int threads, size_t smem, int* per_sm) {
+  std::lock_guard<std::mutex> lk(g_kernel_mu);
+  KernelFacts& f = g_kernels[std::make_pair((const void*)kern, P->device)];
+  if (smem > f.smem) {
+    TRY(set_smem(kern, smem));
+    f.smem = smem;
+  }
+  if (per_sm) {
+    int& n = f.resident[std::make_pair(threads, smem)];
+    if (n < 1) {
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
+      if (n < 1) n = 1;
+    }
+    *per_sm = n;
+  }
+  return PF_OK;
+}
+
 // bytes from p to the end of the workspace holding it: the bound every access is checked
 // against (0 for a pointer outside the workspaces)
 static size_t cap_of(const pf_plan* P, const void* p) {
@@ -450,8 +493,7 @@ static int sm_count(pf_plan* P) {
 template <typename K>
 static pf_status persistent_grid(pf_plan* P, K kern, size_t smem, long long ntiles, unsigned* grid) {
   int per = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kThreads, smem));
-  if (per < 1) per = 1;
+  TRY(kernel_ready(P, kern, kThreads, smem, &per));
   if (P->grid_cap > 0 && P->grid_cap < per) per = P->grid_cap;
   long long g = (long long)per * sm_count(P);
   if (g > ntiles) g = ntiles;
@@ -619,6 +661,16 @@ static pf_status spectrum_alloc(pf_plan* P) {
   return PF_OK;
 }
 
+// bytes of work array 0 that a realization needs (gen_r2c, gen_dft, gen_dctdst)
+static size_t gen_ws_bytes(const pf_plan* P) {
+  const Geom& g = P->g;
+  const size_t e = P->desc.precision == PF_PREC_F64 ? sizeof(double2) : sizeof(float2);
+  if (g.dim == 1) return 0;
+  const size_t inner = g.fb == PF_FIELD_R2C ? (size_t)half_pitch(g) * (g.dim == 3 ? g.T[1] : 1)
+                                            : (size_t)g.T[0] * (g.dim == 3 ? g.T[1] : 1);
+  return e * inner * (size_t)g.n[g.dim - 1];
+}
+
 // vals != NULL: the matrix cells were computed by the caller (device array, dimension 0
 // fastest: prod(T_i/2+1) values for the DCT matrix, prod(T_i) otherwise) and replace the
 // covariance evaluation of the first pass; periodization is then the caller's
@@ -658,11 +710,10 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
     TRY(prof_end(P, &rec));
     cl.c.cof = P->cof + 2;
   }
-  void *A = nullptr, *Bw = nullptr;
+  // one work array: every strided pass rewrites its pencils in place
+  void* A = nullptr;
   double2* spec = nullptr;
-  const uint64_t full = g.mb == PF_MATRIX_DFT ? g.N : g.Nc;
-  TRY(workspace(P, 0, full * sizeof(double2), &A));
-  TRY(workspace(P, 1, full * sizeof(double2), &Bw));
+  TRY(workspace(P, 0, g.S * sizeof(double2), &A));
   cl.rowmod = g.T[1];
   cl.mirror = g.mb == PF_MATRIX_DCT;
   if (g.mb == PF_MATRIX_DCT) {
@@ -685,17 +736,15 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
       MirrorLoad<double2> ml{(const double2*)A, (unsigned)T0c, (unsigned)((long long)T0c * D1), 1u,
                              (unsigned)std::min<size_t>(cap_of(P, A) / sizeof(double2), 0xffffffffu), g.T[1]};
       TRY((run_pass<double, false, -1>(P, "spec_c2c_d1", g.T[1], D1, T0c, D2, ml, NoMid(),
-                                                   arr_store<double2>(P, Bw, T0c, (long long)T0c * D1, 1),
+                                                   arr_store<double2>(P, A, T0c, (long long)T0c * D1, 1),
                                                    (double)T0c * D2 * (D1 + D1) * 16.0)));
-      spec = (double2*)Bw;
       if (dim == 3) {
         const long long inner = (long long)T0c * D1;
-        MirrorLoad<double2> m2{(const double2*)Bw, (unsigned)inner, 0u, 1u,
-                               (unsigned)std::min<size_t>(cap_of(P, Bw) / sizeof(double2), 0xffffffffu), g.T[2]};
+        MirrorLoad<double2> m2{(const double2*)A, (unsigned)inner, 0u, 1u,
+                               (unsigned)std::min<size_t>(cap_of(P, A) / sizeof(double2), 0xffffffffu), g.T[2]};
         TRY((run_pass<double, false, -1>(P, "spec_c2c_d2", g.T[2], D2, inner, 1, m2, NoMid(),
                                                      arr_store<double2>(P, A, inner, 0, 1),
                                                      (double)inner * (D2 + D2) * 16.0)));
-        spec = (double2*)A;
       }
     }
   } else if (g.mb == PF_MATRIX_R2C) {
@@ -716,17 +765,15 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
       const long long outer = dim == 3 ? g.T[2] : 1;
       TRY((run_pass<double, false, -1>(P, "spec_c2c_d1", L1, L1o, T0c, outer,
                                                    arr_load<double2>(P, A, T0c, (long long)T0c * L1, 1, L1), NoMid(),
-                                                   arr_store<double2>(P, Bw, T0c, (long long)T0c * L1o, 1),
+                                                   arr_store<double2>(P, A, T0c, (long long)T0c * L1o, 1),
                                                    (double)T0c * outer * (L1 + L1o) * 16.0)));
-      spec = (double2*)Bw;
       if (dim == 3) {
         const int L2 = g.T[2], L2o = dct ? g.T[2] / 2 + 1 : g.T[2];
         const long long inner = (long long)T0c * L1o;
         TRY((run_pass<double, false, -1>(P, "spec_c2c_d2", L2, L2o, inner, 1,
-                                                     arr_load<double2>(P, Bw, inner, 0, 1, L2), NoMid(),
+                                                     arr_load<double2>(P, A, inner, 0, 1, L2), NoMid(),
                                                      arr_store<double2>(P, A, inner, 0, 1),
                                                      (double)inner * (L2 + L2o) * 16.0)));
-        spec = (double2*)A;
       }
     }
   } else {  // DFT matrix: complex torus, every axis complex (dftmatrixbackend.hh:209-238)
@@ -739,17 +786,13 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
       TRY((run_pass<double, true, -1>(P, "spec_c2c_d0", g.T[0], g.T[0], rows, 1, cl, NoMid(),
                                   arr_store<double2>(P, A, 1, 0, g.T[0]), rows * g.T[0] * 16.0)));
     spec = (double2*)A;
-    void* src = A;
-    void* dst = Bw;
     long long inner = g.T[0];
     for (int ax = 1; ax < dim; ax++) {
       const int L = g.T[ax];
       long long outer = (long long)(g.N / (uint64_t)inner / (uint64_t)L);
       TRY((run_pass<double, false, -1>(P, ax == 1 ? "spec_c2c_d1" : "spec_c2c_d2", L, L, inner, outer,
-                                   arr_load<double2>(P, src, inner, inner * L, 1, L), NoMid(),
-                                   arr_store<double2>(P, dst, inner, inner * L, 1), (double)g.N * 32.0)));
-      spec = (double2*)dst;
-      std::swap(src, dst);
+                                   arr_load<double2>(P, A, inner, inner * L, 1, L), NoMid(),
+                                   arr_store<double2>(P, A, inner, inner * L, 1), (double)g.N * 32.0)));
       inner *= L;
     }
   }
@@ -791,17 +834,17 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
   double mn;
   memcpy(&mn, &b, 8);
   P->stats.smallest = mn;
-  // release the FP64 spectrum workspaces: they are the largest buffers of the plan
-  // (borrowed ones belong to the caller: an ensemble lends one pair to all its fields)
+  // The work array stays for the realizations' first pass and the next build (a loop over
+  // covariance parameters), unless it is larger than they need: the R2C and DFT matrices' is the
+  // largest buffer of the plan and is released.  A borrowed one belongs to the caller (an ensemble
+  // lends one to all its fields).
   if (P->borrowed_ws) {
-    P->ws[0] = P->ws[1] = nullptr;
-    P->ws_bytes[0] = P->ws_bytes[1] = 0;
+    P->ws[0] = nullptr;
+    P->ws_bytes[0] = 0;
     P->borrowed_ws = false;
-  } else {
+  } else if (P->ws_bytes[0] > gen_ws_bytes(P) + gen_ws_bytes(P) / 8) {
     dfree(P, &P->ws[0], P->ws_bytes[0]);
     P->ws_bytes[0] = 0;
-    dfree(P, &P->ws[1], P->ws_bytes[1]);
-    P->ws_bytes[1] = 0;
   }
   if (P->stats.negative > 0 && !d->approximate) {
     P->have_spec = false;
@@ -811,16 +854,45 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
   return PF_OK;
 }
 
-// reads and clears the kernels' bounds-violation flag (synchronizes the stream)
+// the devices' error words (pf_kernels.cuh), host and device view; they live until the process exits
+struct ErrorWords {
+  volatile unsigned* host = nullptr;
+};
+static std::mutex g_err_words_mu;
+static std::map<int, ErrorWords> g_err_words;
+
+static pf_status error_words(int device, volatile unsigned** out) {
+  std::lock_guard<std::mutex> lk(g_err_words_mu);
+  ErrorWords& w = g_err_words[device];
+  if (!w.host) {
+    void *h = nullptr, *d = nullptr;
+    cudaError_t e = cudaHostAlloc(&h, 64, cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess) {
+      memset(h, 0, 64);
+      e = cudaHostGetDevicePointer(&d, h, 0);
+      if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_error_words, &d, sizeof(d));
+      if (e != cudaSuccess) cudaFreeHost(h);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(e == cudaErrorMemoryAllocation ? PF_ERR_OOM : PF_ERR_CUDA, "error words of device %d: %s", device,
+                  cudaGetErrorString(e));
+    }
+    w.host = (volatile unsigned*)h;
+  }
+  *out = w.host;
+  return PF_OK;
+}
+
+// waits for the stream, then reads and clears the device's error words
 static pf_status check_bounds(pf_plan* P, pf_status st) {
-  unsigned int flag = 0;
-  CK(cudaMemcpyFromSymbolAsync(&flag, g_bounds_error, sizeof(flag), 0, cudaMemcpyDeviceToHost, P->stream));
   CK(cudaStreamSynchronize(P->stream));
-  if (flag) {
-    const unsigned int zero = 0;
-    CK(cudaMemcpyToSymbolAsync(g_bounds_error, &zero, sizeof(zero), 0, cudaMemcpyHostToDevice, P->stream));
-    CK(cudaStreamSynchronize(P->stream));
-    if (flag & 2u) return fail(PF_ERR_TIMEOUT, "a kernel's bounded wait for its tile copies gave up");
+  volatile unsigned* const w = P->err_words;
+  if (w[0] | w[1]) {
+    const bool timeout = w[1] != 0;
+    w[0] = 0u;
+    w[1] = 0u;
+    if (timeout) return fail(PF_ERR_TIMEOUT, "a kernel's bounded wait for its tile copies gave up");
     return fail(PF_ERR_CUDA, "internal error: a kernel computed an index outside its buffer (access skipped)");
   }
   return st;
@@ -1429,10 +1501,15 @@ pf_status pf_plan_create(const pf_field_desc* desc, pf_plan** plan) {
     cudaGetLastError();
     return fail(PF_ERR_CUDA, "no CUDA device available (%s)", cudaGetErrorString(e));
   }
+  int device = 0;
+  cudaGetDevice(&device);
+  volatile unsigned* words = nullptr;
+  TRY(error_words(device, &words));
   pf_plan* P = new pf_plan();
   P->desc = *desc;
   P->g = g;
-  cudaGetDevice(&P->device);
+  P->device = device;
+  P->err_words = words;
   e = cudaStreamCreateWithFlags(&P->own, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete P;

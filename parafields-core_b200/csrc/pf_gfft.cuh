@@ -284,9 +284,12 @@ __device__ __forceinline__ void g_dft(CV<R>* v) {
   }
 }
 
-// radices of the kernels with fused ends, and of the shared stages
-#define PF_G_FUSED_RADICES(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8)
-#define PF_G_RADICES(X) X(1) PF_G_FUSED_RADICES(X) X(11) X(13)
+// radices of the kernels with fused ends; of the shared stages, those that would make the common
+// ones spill registers apart (with the error words' address in constant memory: 32 fields, mostly Bluestein
+// lengths, 715 -> 664 us)
+#define PF_G_COMMON_RADICES(X) X(2) X(3) X(4) X(5) X(6) X(8)
+#define PF_G_RARE_RADICES(X) X(1) X(7) X(11) X(13)
+#define PF_G_FUSED_RADICES(X) PF_G_COMMON_RADICES(X) X(7)
 
 // ---------------------------------------------------------------------------
 // pass descriptor
@@ -535,14 +538,25 @@ __device__ __forceinline__ void g_stage_r(const GArgs<T>& a, const GStage& g) {
   __syncthreads();
 }
 template <typename T, bool ROWS, int KIND>
+__device__ __noinline__ void g_stage_rare(const GArgs<T>& a, int s) {
+  const GStage& g = a.st[s];
+  switch (g.R) {
+#define PF_G_CASE(RR) \
+  case RR: g_stage_r<T, ROWS, KIND, RR>(a, g); break;
+    PF_G_RARE_RADICES(PF_G_CASE)
+#undef PF_G_CASE
+    default: break;
+  }
+}
+template <typename T, bool ROWS, int KIND>
 __device__ __noinline__ void g_stage(const GArgs<T>& a, int s) {
   const GStage& g = a.st[s];
   switch (g.R) {
 #define PF_G_CASE(RR) \
   case RR: g_stage_r<T, ROWS, KIND, RR>(a, g); break;
-    PF_G_RADICES(PF_G_CASE)
+    PF_G_COMMON_RADICES(PF_G_CASE)
 #undef PF_G_CASE
-    default: break;
+    default: g_stage_rare<T, ROWS, KIND>(a, s);
   }
 }
 
@@ -941,7 +955,7 @@ __global__ void __launch_bounds__(kGThreads, 1)
   if constexpr (FUSED) {
     if (!(GIn<T, MODE, Ld>::fits(a, ld, last, io) && GOut<T, MODE, St>::fits(a, st, last, io) &&
           GFac<T>::fits(a, mid, last, io))) {  // the same for all threads of the block
-      if (threadIdx.x == 0) atomicOr(&g_bounds_error, 1u);
+      if (threadIdx.x == 0) report_error(1u);
       return;
     }
   }
@@ -1006,7 +1020,7 @@ __global__ void __launch_bounds__(kGThreads, 1)
         // the block size is a multiple of B: a thread keeps its slot
         const int b = threadIdx.x & (B - 1), dn = nt >> a.lgB, h = a.L / 2;
         if (!GNoise<T>(a, ld, last, last, io).fits(a)) {  // the same for all threads of the block
-          if (threadIdx.x == 0) atomicOr(&g_bounds_error, 1u);
+          if (threadIdx.x == 0) report_error(1u);
           return;
         }
         const GNoise<T> g(a, ld, p0 + PAIR * b, last, io);

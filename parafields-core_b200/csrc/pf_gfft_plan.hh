@@ -41,7 +41,7 @@ struct GSched {
 };
 static std::mutex g_sched_mu;
 
-static GSched g_schedule_locked(int N) {
+static const GSched& g_schedule_locked(int N) {  // entries stay in place
   static std::map<int, GSched> cache;
   auto it = cache.find(N);
   if (it != cache.end()) return it->second;
@@ -53,10 +53,9 @@ static GSched g_schedule_locked(int N) {
     std::vector<int> cur;
     g_search(N, 13, cur, 0., s.r, s.cost);
   }
-  cache[N] = s;
-  return s;
+  return cache[N] = s;
 }
-static GSched g_schedule(int N) {
+static const GSched& g_schedule(int N) {
   std::lock_guard<std::mutex> lk(g_sched_mu);
   return g_schedule_locked(N);
 }
@@ -76,7 +75,7 @@ static int g_blue_length(int L) {
     for (int p : {2, 3, 5, 7})
       while (x % p == 0) x /= p;
     if (x != 1) continue;
-    const GSched s = g_schedule_locked(n);
+    const GSched& s = g_schedule_locked(n);
     if (s.r.size() >= 2 && s.cost * n < bc) {
       bc = s.cost * n;
       best = n;
@@ -122,6 +121,7 @@ static void g_tile(int slots, const std::vector<int>& r, bool rows, bool direct,
   // work items of the widest step
   const long long wide = (long long)B * slots / (direct ? *std::min_element(r.begin(), r.end()) : 2);
   double best = 1e300;
+  *nt_out = 32;
   for (int nt = 32; nt <= top && nt < wide + 32; nt += 32) {
     double t = 0.;
     for (int R : r) t += (double)(((long long)B * (slots / R) + nt - 1) / nt) * (R + 4);

@@ -13,19 +13,26 @@ namespace pf {
 #endif
 constexpr int kThreads = PF_THREADS;
 
-// Set by any functor whose computed index falls outside its buffer; the access is
-// skipped instead of performed, and the host turns the flag into an error.
-__device__ unsigned int g_bounds_error;
+// Error words of the device, in host memory the device can write (set when the first plan is
+// created, check_bounds in pf_capi.cu): [0] an index outside its buffer (the access is skipped),
+// [1] a bounded wait gave up.  The host reads them after the stream has drained, without a copy.
+__constant__ unsigned int* g_error_words;
+
+// bit 1: index outside its buffer; bit 2: a wait gave up
+__device__ __forceinline__ void report_error(unsigned bits) {
+  if (bits & 1u) *(volatile unsigned int*)g_error_words = 1u;
+  if (bits & 2u) *(volatile unsigned int*)(g_error_words + 1) = 1u;
+}
 
 __device__ __forceinline__ bool in_bounds(long long i, long long n) {
   if (i >= 0 && i < n) return true;
-  atomicOr(&g_bounds_error, 1u);
+  report_error(1u);
   return false;
 }
 // 32-bit element indices (every buffer of a plan holds fewer than 2^32 elements)
 __device__ __forceinline__ bool in_bounds32(unsigned i, unsigned n) {
   if (i < n) return true;
-  atomicOr(&g_bounds_error, 1u);
+  report_error(1u);
   return false;
 }
 

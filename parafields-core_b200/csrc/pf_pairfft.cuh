@@ -220,7 +220,7 @@ __device__ __forceinline__ void p2_copy_table(float4* dst, const float4* __restr
 
 // bit 1: an index outside its buffer (access skipped); bit 2: a bounded wait gave up
 __device__ __forceinline__ void p2_report(unsigned bad) {
-  if (bad) atomicOr(&g_bounds_error, bad);
+  if (bad) report_error(bad);
 }
 
 // ---------------------------------------------------------------------------
@@ -442,7 +442,7 @@ __global__ void k_export_noise(NoiseExport e, double* __restrict__ out) {
       }
     }
   }
-  if (bad) atomicOr(&g_bounds_error, 1u);
+  if (bad) report_error(1u);
 }
 
 template <int DIM, int LAYOUT, bool TRANSP>
