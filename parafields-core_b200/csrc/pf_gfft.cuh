@@ -285,7 +285,7 @@ __device__ __forceinline__ void g_dft(CV<R>* v) {
 }
 
 // radices of the kernels with fused ends; of the shared stages, those that would make the common
-// ones spill registers apart (with the error words' address in constant memory: 32 fields, mostly Bluestein
+// ones spill registers apart (with the error words' address in constant memory: 32 uneven 2D fields, mostly Bluestein
 // lengths, 715 -> 664 us)
 #define PF_G_COMMON_RADICES(X) X(2) X(3) X(4) X(5) X(6) X(8)
 #define PF_G_RARE_RADICES(X) X(1) X(7) X(11) X(13)
@@ -320,6 +320,7 @@ struct GArgs {
   int M1p;             // padded distance of the first stage's sub-blocks
   int pitch;           // slots of one row
   int np, tpo;         // pencils (per outer block), tiles per outer block
+  int args_at;         // slot of shared memory that holds a copy of these for the shared stages; 0: none
   unsigned mL, mLh, mLout;  // divisors L, L/2, outputs per row of the post-processing
   const W* tw;         // stage twiddles
   const W* twT;        // real rows: exp(-2 pi i m / 2L), m < L
@@ -928,7 +929,6 @@ __global__ void __launch_bounds__(kGThreads, 1)
     k_g(const __grid_constant__ GArgs<T> a, const __grid_constant__ Ld ld, const __grid_constant__ Mid mid,
         const __grid_constant__ St st) {
   chain_start();
-  chain_wait();
   using R_ = typename GT<T>::R;
   using V = CV<R_>;
   constexpr int PAIR = GT<T>::PAIR;
@@ -936,6 +936,16 @@ __global__ void __launch_bounds__(kGThreads, 1)
   static_assert(!Mid::active || (MODE == 0 && SIGN < 0), "the fused pass is forward, factor, backward");
   extern __shared__ __align__(16) unsigned char g_smem[];
   V* const sm = reinterpret_cast<V*>(g_smem);
+  // the shared stages take their arguments by reference: from shared memory, the kernel's
+  // parameters being slow to read through a pointer
+  const GArgs<T>* sa = &a;
+  if (!FUSED && a.args_at) {
+    int* const d = reinterpret_cast<int*>(sm + a.args_at);
+    for (int i = threadIdx.x; i < (int)(sizeof(a) / 4); i += blockDim.x) d[i] = reinterpret_cast<const int*>(&a)[i];
+    sa = reinterpret_cast<const GArgs<T>*>(sm + a.args_at);
+    __syncthreads();
+  }
+  chain_wait();
   const GTile<T, ROWS> ti{a};
   const int nt = blockDim.x;
   const int B = a.B, np = a.np;
@@ -1041,7 +1051,7 @@ __global__ void __launch_bounds__(kGThreads, 1)
         sm[ti.slot0(b) + ti.place(n)] = enter(n, fetch(p0 + PAIR * b, n));
       }
     __syncthreads();
-    g_stage<T, ROWS, 0>(a, 0);
+    g_stage<T, ROWS, 0>(*sa, 0);
   } else {
     auto stage_first = [&](auto rc) {
       constexpr int R = decltype(rc)::value;
@@ -1075,13 +1085,13 @@ __global__ void __launch_bounds__(kGThreads, 1)
   // ---- any length ------------------------------------------------------------------------
   if constexpr (!FUSED) {
     auto forward = [&]() {  // the forward transform, and for Bluestein the convolution
-      for (int s = 1; s < S - 1; s++) g_stage<T, ROWS, 1>(a, s);
+      for (int s = 1; s < S - 1; s++) g_stage<T, ROWS, 1>(*sa, s);
       if (blue) {
-        g_stage<T, ROWS, 5>(a, S - 1);
-        for (int s = S - 2; s >= 1; s--) g_stage<T, ROWS, 3>(a, s);
-        g_stage<T, ROWS, 4>(a, 0);
+        g_stage<T, ROWS, 5>(*sa, S - 1);
+        for (int s = S - 2; s >= 1; s--) g_stage<T, ROWS, 3>(*sa, s);
+        g_stage<T, ROWS, 4>(*sa, 0);
       } else if (S > 1) {
-        g_stage<T, ROWS, 2>(a, S - 1);
+        g_stage<T, ROWS, 2>(*sa, S - 1);
       }
     };
     // output j < L of forward(): with Bluestein's algorithm in the order of the inputs
@@ -1100,12 +1110,12 @@ __global__ void __launch_bounds__(kGThreads, 1)
       }
       __syncthreads();
       if (blue) {  // the backward transform is a second convolution
-        g_stage<T, ROWS, 0>(a, 0);
+        g_stage<T, ROWS, 0>(*sa, 0);
         forward();
       } else {
-        if (S > 1) g_stage<T, ROWS, 2>(a, S - 1);
-        for (int s = S - 2; s >= 1; s--) g_stage<T, ROWS, 3>(a, s);
-        g_stage<T, ROWS, 4>(a, 0);
+        if (S > 1) g_stage<T, ROWS, 2>(*sa, S - 1);
+        for (int s = S - 2; s >= 1; s--) g_stage<T, ROWS, 3>(*sa, s);
+        g_stage<T, ROWS, 4>(*sa, 0);
       }
       const int n1 = a.Lout < a.L ? a.Lout : a.L;
       for (int u = threadIdx.x; u < B * n1; u += nt) {
@@ -1135,7 +1145,13 @@ __global__ void __launch_bounds__(kGThreads, 1)
       }
     }
     if constexpr (MODE == 1) {
-      g_stage<T, ROWS, 2>(a, S - 1);
+      switch (a.st[S - 1].R) {
+#define PF_G_CASE(RR) \
+  case RR: g_stage_r<T, ROWS, 2, RR>(a, a.st[S - 1]); break;
+        PF_G_FUSED_RADICES(PF_G_CASE)
+#undef PF_G_CASE
+        default: break;
+      }
     } else {
       // last stage: outputs to the store, or through the factor and the first stage of the
       // backward transform
@@ -1213,9 +1229,9 @@ __global__ void __launch_bounds__(kGThreads, 1)
     }
   }
 
-  if constexpr (MODE == 1) {  // split of the half-length transform: X_k from Z_k and Z_(L-k)
+  if constexpr (MODE == 1) {  // split of the half-length transform: X_k and X_(L-k) from Z_k and Z_(L-k)
     const R_ half = g_const<R_>(0.5);
-    const int n1 = a.Lout;
+    const int n1 = a.L / 2 + 1;
     auto z = [&](int b, int k) -> V {
       const int at = ti.slot0(b) + (blue ? ti.place(k) : ti.place_out(k));
       return blue ? v_mul(v_swap(sm[at]), __ldg(a.chirp + k)) : sm[at];
@@ -1223,12 +1239,15 @@ __global__ void __launch_bounds__(kGThreads, 1)
     for (int u = threadIdx.x; u < B * n1; u += nt) {
       int b, k;
       ti.split(u, n1, a.mLout, b, k);
-      const V zk = z(b, k == a.L ? 0 : k), zm = z(b, k == 0 ? 0 : a.L - k);
+      const V zk = z(b, k), zm = z(b, k == 0 ? 0 : a.L - k);
+      // e = (Z_k + conj Z_(L-k)) / 2, o = (Z_k - conj Z_(L-k)) / 2, t = -i o exp(-pi i k / L):
+      // X_k = e + t, X_(L-k) = conj(e - t)
       const V e = {g_mul(half, g_add(zk.re, zm.re)), g_mul(half, g_sub(zk.im, zm.im))};
       const V o = {g_mul(half, g_sub(zk.re, zm.re)), g_mul(half, g_add(zk.im, zm.im))};
-      const V oi = {o.im, g_neg(o.re)};
-      const V x = k == a.L ? v_sub(e, oi) : v_add(e, v_mul(oi, __ldg(a.twT + k)));
-      g_store(st, p0 + PAIR * b, np, k, 0, x);
+      const V t = v_mul(V{o.im, g_neg(o.re)}, __ldg(a.twT + k));
+      const int p = p0 + PAIR * b;
+      g_store(st, p, np, k, 0, v_add(e, t));
+      if (2 * k != a.L) g_store(st, p, np, a.L - k, 0, V{g_sub(e.re, t.re), g_sub(t.im, e.im)});
     }
   }
 }

@@ -165,6 +165,6 @@ static void g_fill(GArgs<T>& a, const GSched& sc, int N, int L, int Lout, int mo
   a.pitch = a.M1p * R1;
   a.mL = g_magic(L);
   a.mLh = g_magic(L / 2);
-  // outputs per slot of the store phase
-  a.mLout = g_magic(mode == 2 ? (Lout + 1) / 2 : (mid ? std::min(Lout, L) : Lout));
+  // items per slot of the store phase
+  a.mLout = g_magic(mode == 1 ? L / 2 + 1 : (mode == 2 ? (Lout + 1) / 2 : (mid ? std::min(Lout, L) : Lout)));
 }

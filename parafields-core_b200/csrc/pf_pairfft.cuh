@@ -943,68 +943,6 @@ __global__ void __launch_bounds__(kP2Threads, 2)
 }
 
 // ---------------------------------------------------------------------------
-// Complex-to-real rows (2L reals from L+1 complex, FFTW c2r semantics: Im of the DC
-// and Nyquist inputs ignored), rows p and p+1 per pair, threads along the row.
-// Store(p, m, x0, x1) receives reals 2m and 2m+1 of row p.
-// ---------------------------------------------------------------------------
-template <int L, class St>
-__global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2R)
-    kp2_c2r(const float4* __restrict__ twg, long long ntiles, int Lout, P2RowLoad ld, St st) {
-  chain_start();
-  using G = P2Geom<L>;
-  extern __shared__ __align__(16) float4 p2_smem[];
-  float4* buf = p2_smem;
-  float4* tw = p2_smem + G::Q * G::PLQ;
-  const float4* twT = tw + G::NTW;  // exp(+2 pi i m / 2L), m < L
-  p2_copy_table(tw, twg, G::NTW + L);
-  chain_wait();
-  __syncthreads();
-  const int u = threadIdx.x % G::TP, q = threadIdx.x / G::TP;
-  unsigned bad = 0;
-  [[maybe_unused]] double acc = 0.;  // St::kDot: this thread's share of the dot product
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int p = (int)tile * G::NP + 2 * q;
-    P2 v[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int m = u + r * G::TP;
-      float2 xa = ld.one(p, m, bad), xb = ld.one(p + 1, m, bad);
-      float2 ya = ld.one(p, L - m, bad), yb = ld.one(p + 1, L - m, bad);
-      if (m == 0) {
-        xa.y = 0.f;
-        xb.y = 0.f;
-        ya.y = 0.f;
-        yb.y = 0.f;
-      }
-      const P2 X = p2_ab(xa, xb), Y = p2_ab(ya, yb);
-      // s = X + conj(Y), d = X - conj(Y), t = d w, Z = s + i t
-      const P2 s = {f2add(X.re, Y.re), f2sub(X.im, Y.im)};
-      const P2 d = {f2sub(X.re, Y.re), f2add(X.im, Y.im)};
-      const P2 t = ptw(d, twT[m]);
-      v[r] = {f2sub(s.re, t.im), f2add(s.im, t.re)};
-    }
-    p2_transform<L, +1>(v, buf, tw, u, q, [&](int m, const P2& z) {
-      if (2 * m < Lout) {
-        st.store(p, m, z, bad);
-        if constexpr (St::kDot) acc += st.dot(p, m, z);
-      }
-    });
-  }
-  if constexpr (St::kDot) {  // a . out over the stored values, finished by the last block
-    __shared__ double shd[32];
-    acc = block_sum(acc, shd);
-    if (cg_last_block(acc, st.part, st.cnt)) {
-      const double t = cg_sum_partials(st.part, shd);
-      if (threadIdx.x == 0) {
-        *st.sdst = t;
-        *st.cnt = 0u;
-      }
-    }
-  }
-  p2_report(bad);
-}
-
-// ---------------------------------------------------------------------------
 // Complex-to-real rows with the rows staged by bulk copies.  A tile's NP rows are adjacent
 // in memory (row stride `rowstride` complex, 16-byte multiple), so one cp.async.bulk per
 // tile moves them into shared memory, completion counted on an mbarrier; two tile buffers
@@ -1123,7 +1061,6 @@ __global__ void __launch_bounds__(kP2Threads, 2)
 template <typename O>
 struct P2FieldStoreT {
   using O2 = typename std::conditional<sizeof(O) == 8, double2, float2>::type;
-  static constexpr bool kDot = false;
   O* out;
   int n0;
   int transform;
@@ -1159,30 +1096,6 @@ struct P2FieldStoreT {
   }
 };
 using P2FieldStore = P2FieldStoreT<float>;
-
-// FP64 rows of the matvec's output that also accumulate dv . out over the stored values
-// (the CG's d . A d); kp2_c2r finishes the sum with the last-block reduction into *sdst.
-// Every output element is stored exactly once, so every product enters once; the order of
-// the sum is fixed by the kernel's static tile order.
-struct P2FieldDotStore : P2FieldStoreT<double> {
-  static constexpr bool kDot = true;
-  const double* dv;
-  double* part;   // one partial per CTA
-  unsigned* cnt;  // ticket, 0 between kernels
-  double* sdst;
-  __device__ __forceinline__ double dot1(int p, int m, float a, float b) const {
-    if (p >= np) return 0.;
-    const unsigned i = (unsigned)p * (unsigned)n0 + 2u * (unsigned)m;
-    const bool two = 2 * m + 1 < Lout;
-    if (i + (two ? 1u : 0u) >= n) return 0.;
-    double r = dv[i] * (double)a;
-    if (two) r += dv[i + 1] * (double)b;
-    return r;
-  }
-  __device__ __forceinline__ double dot(int p, int m, const P2& z) const {
-    return dot1(p, m, z.re.x, z.im.x) + dot1(p + 1, m, z.re.y, z.im.y);
-  }
-};
 
 // ---------------------------------------------------------------------------
 // Real-to-complex rows (L+1 complex from 2L reals, FFTW r2c semantics), the forward
