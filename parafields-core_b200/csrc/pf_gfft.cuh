@@ -32,9 +32,9 @@
 // issue slots are 35-55% busy, HBM below 45%.  Measured on one B200 against the passes it replaced
 // (two ping-pong buffers, runtime divisions per element, 2 CTAs per SM; compile-time schedules
 // for 11 lengths; radix-2 Bluestein), us: 100^3 FP64 realization, passes of 200, 200 and 100
-// points, 116 / 44 / 34 -> 75 / 21 / 17; FP64 product on 128^3 (256 points) 287 -> 225, its fused
-// pass 148 -> 85; FP32 product on 150 x 100 x 75 279 -> 100; 32 uneven 2D fields, mostly
-// Bluestein lengths, 1330 -> 730; FP64 covariance rows of a 256^3 DCT spectrum 1277 -> 546.
+// points, 116 / 44 / 34 -> 67 / 21 / 17; FP64 product on 128^3 (256 points) 287 -> 193, its fused
+// pass 148 -> 85; FP32 product on 150 x 100 x 75 279 -> 80; 32 uneven 2D fields, mostly
+// Bluestein lengths, 1330 -> 638; FP64 covariance rows of a 256^3 DCT spectrum 1277 -> 546.
 //
 // Layout of a tile of B slots: strided passes keep the B adjacent pencils together (element n of
 // slot b at n B + b); row passes keep rows together (b * pitch + n), the R1 sub-blocks of a row

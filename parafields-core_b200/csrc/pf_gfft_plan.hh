@@ -97,7 +97,8 @@ constexpr size_t kGSmem = 227 * 1024;
 
 // Slots per tile and threads.  Strided tiles take 8 slots (128-byte row segments) while three
 // of them fit on an SM, fewer for longer pencils but at least 2 (one 32-byte sector) while two
-// fit; row tiles about 1024 elements (2048 where the loader computes its values).  Fewer slots
+// fit; row tiles up to 1024 elements, 2048 where the loader computes its values (192-point FP32 rows
+// beside another stream's passes 87 us with 8 pairs per tile, 74 with 4; 128-point rows 15 with 8, 18 with 4).  Fewer slots
 // where the grid would leave SMs idle.  Threads: the count with the least estimated time, which
 // is rounds of butterflies (and of loader pairs) per tile over the tiles that run at once on an SM
 // within 1024 threads, the tile's shared memory and the grid.
@@ -106,7 +107,7 @@ static void g_tile(int slots, const std::vector<int>& r, bool rows, bool direct,
   const size_t per = (size_t)16 * pitch;
   int B = 1;
   if (rows) {
-    while (B < 32 && B * slots < (direct ? 1024 : 2048) && 2 * B * per <= kGSmem / 3) B *= 2;
+    while (B < 32 && 2 * B * slots <= (direct ? 1024 : 2048) && 2 * B * per <= kGSmem / 3) B *= 2;
   } else {
     B = 8;
     while (B > 2 && B * per > kGSmem / 3) B /= 2;

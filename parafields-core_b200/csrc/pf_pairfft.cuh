@@ -31,17 +31,16 @@ constexpr int pick_radix(int m) { return m % 8 == 0 ? 8 : (m % 4 == 0 ? 4 : 2); 
 // resident CTAs per SM the register allocation is sized for (per kernel family).  The
 // strided pass is held to 64 registers (4 CTAs per SM): alone it runs as fast as with 3,
 // and in the two-stream batch its CTAs fit beside the other stream's kernels (256^3
-// Matern-3/2 batch: 0.388 against 0.401 ms per realization).  At 64 registers the
-// complex-to-real pass spills and runs slower alone (0.088 against 0.077 ms) and in the
-// batch, so it keeps 3.
+// Matern-3/2 batch: 0.388 against 0.401 ms per realization).  The real-to-complex rows take 80
+// registers (3 CTAs per SM).
 #ifndef PF_P2_MIN_NOISE
 #define PF_P2_MIN_NOISE 4
 #endif
 #ifndef PF_P2_MIN_C2C
 #define PF_P2_MIN_C2C 4
 #endif
-#ifndef PF_P2_MIN_C2R
-#define PF_P2_MIN_C2R 3
+#ifndef PF_P2_MIN_R2C
+#define PF_P2_MIN_R2C 3
 #endif
 
 struct P2 {
@@ -1195,7 +1194,7 @@ struct P2RowStore {
 };
 
 template <int L, class Ld>
-__global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_C2R)
+__global__ void __launch_bounds__(kP2Threads, PF_P2_MIN_R2C)
     kp2_r2c(const float4* __restrict__ twg, long long ntiles, Ld ld, P2RowStore st) {
   chain_start();
   using G = P2Geom<L>;
