@@ -1228,6 +1228,8 @@ __device__ __forceinline__ double dkey_value(unsigned long long k) {
 // keys[1] = max key of those with norm > 1 within ext/T of half the torus on some axis.
 __global__ void __launch_bounds__(kThreads) k_cofold_stats(CovParams c, int C0, int C1, int C2,
                                                            unsigned long long* keys) {
+  chain_start();
+  chain_wait();  // the keys' initial values
   unsigned long long mn = ~0ull, mx = 0ull;
   const uint64_t n = (uint64_t)C0 * C1 * C2;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -1264,6 +1266,8 @@ __global__ void __launch_bounds__(kThreads) k_cofold_stats(CovParams c, int C0, 
 // offset = beta - integral_alpha^beta sigmoid (matrix.hh:947-972); cof = {active, alpha,
 // beta, offset}; inactive (identity) when either set of cells is empty
 __global__ void k_cofold_finish(CovParams c, double max_factor, const unsigned long long* keys, double* cof) {
+  chain_start();
+  chain_wait();  // the atomics of k_cofold_stats
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   if (keys[0] == ~0ull || keys[1] == 0ull) {
     cof[0] = 0.;
