@@ -707,10 +707,15 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
     TRY(prof_end(P, &rec));
     cl.c.cof = P->cof + 2;
   }
-  // one work array: every strided pass rewrites its pencils in place
+  // One work array: every strided pass rewrites its pencils in place.  Where a realization's first
+  // pass takes about as much, the array is allocated at the larger of both sizes and kept, so that
+  // the first realization neither frees nor allocates it: 512^2 FP64 43 us, where it took 645 with an array
+  // of the spectrum's own size, a few percent too small, and 414 with the array released here.
   void* A = nullptr;
   double2* spec = nullptr;
-  TRY(workspace(P, 0, g.S * sizeof(double2), &A));
+  const size_t need = g.S * sizeof(double2), gen = gen_ws_bytes(P);
+  const bool keep = !P->borrowed_ws && need <= gen + gen / 8;
+  TRY(workspace(P, 0, keep ? std::max(need, gen) : need, &A));
   cl.rowmod = g.T[1];
   cl.mirror = g.mb == PF_MATRIX_DCT;
   if (g.mb == PF_MATRIX_DCT) {
@@ -832,14 +837,14 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
   memcpy(&mn, &b, 8);
   P->stats.smallest = mn;
   // The work array stays for the realizations' first pass and the next build (a loop over
-  // covariance parameters), unless it is larger than they need: the R2C and DFT matrices' is the
-  // largest buffer of the plan and is released.  A borrowed one belongs to the caller (an ensemble
-  // lends one to all its fields).
+  // covariance parameters), unless it is larger than a realization needs: the R2C and DFT matrices'
+  // is the largest buffer of the plan and is released.  A borrowed one belongs to the caller (an
+  // ensemble lends one to all its fields).
   if (P->borrowed_ws) {
     P->ws[0] = nullptr;
     P->ws_bytes[0] = 0;
     P->borrowed_ws = false;
-  } else if (P->ws_bytes[0] > gen_ws_bytes(P) + gen_ws_bytes(P) / 8) {
+  } else if (!keep) {
     dfree(P, &P->ws[0], P->ws_bytes[0]);
     P->ws_bytes[0] = 0;
   }
