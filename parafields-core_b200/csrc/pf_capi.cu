@@ -225,6 +225,8 @@ struct pf_plan {
   ScanOut* scan = nullptr;
   double* cof = nullptr;  // cofold: 2 keys, then {active, alpha, beta, offset}
   // workspaces
+  // 0: the spectrum, the first pass of realizations, products where it is large enough; 1: the
+  // second array of 3D realizations and products; 2: products that array 0 is too small for
   void* ws[3] = {nullptr, nullptr, nullptr};
   size_t ws_bytes[3] = {0, 0, 0};
   double* noise_dev = nullptr;
@@ -247,7 +249,7 @@ struct pf_plan {
   uint64_t bytes_held = 0;
   // device word mixed into the noise counters (ensembles replaying a captured graph)
   const unsigned* epoch = nullptr;
-  // ws[0..1] are lent by an ensemble for one spectrum build (not freed by the plan)
+  // ws[0] is lent by an ensemble for one spectrum build (not freed by the plan)
   bool borrowed_ws = false;
   // learned preconditioner of the residual-mode CG (pf_plan_set_preconditioner), not owned
   pf_learned* learned = nullptr;
@@ -321,6 +323,19 @@ static pf_status ensure(pf_plan* P, void** p, size_t* cap, size_t bytes) {
 static pf_status workspace(pf_plan* P, int i, size_t bytes, void** out) {
   TRY(ensure(P, &P->ws[i], &P->ws_bytes[i], bytes));
   *out = P->ws[i];
+  return PF_OK;
+}
+
+// Work arrays of a product: the largest (padded spectrum, `big` bytes) and, in 3D, the rows' spectrum
+// (`small` bytes, else 0).  The largest takes array 0, which realizations and spectra use, so that a
+// plan that only multiplies holds no array it does not read; where array 0 is too small for it (FP64
+// products of an FP32 plan) the rows' spectrum takes array 0.  Array 0 is not replaced by a
+// larger one: the first FP64 product of a 128^3 FP32 plan takes 1.00 ms, and 1.57 when it is.
+static pf_status product_workspaces(pf_plan* P, size_t elem, size_t big, size_t small, void** b, void** s) {
+  const size_t own = P->desc.precision == PF_PREC_F64 ? sizeof(double2) : sizeof(float2);
+  const int ib = (P->ws[0] ? P->ws_bytes[0] >= big : elem <= own) ? 0 : 2;
+  TRY(workspace(P, ib, big, b));
+  if (small) TRY(workspace(P, ib == 2 && P->ws[0] && P->ws_bytes[0] >= small ? 0 : 1, small, s));
   return PF_OK;
 }
 
@@ -715,6 +730,7 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
   double2* spec = nullptr;
   const size_t need = g.S * sizeof(double2), gen = gen_ws_bytes(P);
   const bool keep = !P->borrowed_ws && need <= gen + gen / 8;
+  const size_t had = P->ws_bytes[0];
   TRY(workspace(P, 0, keep ? std::max(need, gen) : need, &A));
   cl.rowmod = g.T[1];
   cl.mirror = g.mb == PF_MATRIX_DCT;
@@ -836,15 +852,15 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
   double mn;
   memcpy(&mn, &b, 8);
   P->stats.smallest = mn;
-  // The work array stays for the realizations' first pass and the next build (a loop over
-  // covariance parameters), unless it is larger than a realization needs: the R2C and DFT matrices'
-  // is the largest buffer of the plan and is released.  A borrowed one belongs to the caller (an
-  // ensemble lends one to all its fields).
+  // The work array stays for the realizations' first pass, the products and the next build (a loop
+  // over covariance parameters), unless this build made it larger than they need: the R2C and DFT
+  // matrices' is the largest buffer of the plan and is released.  A borrowed one belongs to the
+  // caller (an ensemble lends one to all its fields).
   if (P->borrowed_ws) {
     P->ws[0] = nullptr;
     P->ws_bytes[0] = 0;
     P->borrowed_ws = false;
-  } else if (!keep) {
+  } else if (!keep && P->ws_bytes[0] > had) {
     dfree(P, &P->ws[0], P->ws_bytes[0]);
     P->ws_bytes[0] = 0;
   }
@@ -1215,7 +1231,7 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
   };
   if (g.dim == 2) {
     void* X1 = nullptr;
-    TRY(workspace(P, 2, sizeof(cx<T>) * (size_t)P0 * g.n[1], &X1));
+    TRY(product_workspaces(P, sizeof(cx<T>), sizeof(cx<T>) * (size_t)P0 * g.n[1], 0, &X1, nullptr));
     TRY(fwd_rows(X1, g.n[1]));
     const double bf1 = (double)T0c * (2.0 * g.n[1] * e + g.T[1] * lb);
     TRY((run_pass<T, false, -1>(P, "mv_fused_d1", g.T[1], g.n[1], T0c, 1, arr_load<cx<T>>(P, X1, P0, 0, 1, g.n[1]), mid,
@@ -1223,8 +1239,8 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
     return inv_rows(X1, g.n[1]);
   }
   void *X1 = nullptr, *X2 = nullptr;
-  TRY(workspace(P, 1, sizeof(cx<T>) * (size_t)P0 * g.n[1] * g.n[2], &X1));
-  TRY(workspace(P, 2, sizeof(cx<T>) * (size_t)P0 * g.T[1] * g.n[2], &X2));
+  TRY(product_workspaces(P, sizeof(cx<T>), sizeof(cx<T>) * (size_t)P0 * g.T[1] * g.n[2],
+                         sizeof(cx<T>) * (size_t)P0 * g.n[1] * g.n[2], &X2, &X1));
   const long long rows = (long long)g.n[1] * g.n[2];
   const long long s2 = (long long)P0 * g.T[1];
   TRY(fwd_rows(X1, rows));
@@ -1271,7 +1287,7 @@ static pf_status matvec_dft(pf_plan* P, int op, const S* in, S* out) {
   const long long rows = (long long)(g.domain / (uint64_t)g.n[0]);
   void *X1 = nullptr, *X2 = nullptr;
   if (g.dim == 2) {
-    TRY(workspace(P, 2, sizeof(cx<T>) * (size_t)g.T[0] * g.n[1], &X1));
+    TRY(product_workspaces(P, sizeof(cx<T>), sizeof(cx<T>) * (size_t)g.T[0] * g.n[1], 0, &X1, nullptr));
     TRY((run_pass<T, true, -1>(P, "mv_dft_d0", g.T[0], g.T[0], rows, 1, fl, NoMid(),
                            arr_store<cx<T>>(P, X1, 1, 0, g.T[0]), (double)rows * (g.n[0] * sizeof(S) + g.T[0] * e))));
     TRY((run_pass<T, false, -1>(P, "mv_dft_fused_d1", g.T[1], g.n[1], g.T[0], 1,
@@ -1282,8 +1298,8 @@ static pf_status matvec_dft(pf_plan* P, int op, const S* in, S* out) {
                              (double)rows * (g.T[0] * e + g.n[0] * sizeof(S)));
   }
   const long long in1 = (long long)g.T[0] * g.T[1];
-  TRY(workspace(P, 1, sizeof(cx<T>) * (size_t)g.T[0] * g.n[1] * g.n[2], &X1));
-  TRY(workspace(P, 2, sizeof(cx<T>) * (size_t)in1 * g.n[2], &X2));
+  TRY(product_workspaces(P, sizeof(cx<T>), sizeof(cx<T>) * (size_t)in1 * g.n[2],
+                         sizeof(cx<T>) * (size_t)g.T[0] * g.n[1] * g.n[2], &X2, &X1));
   TRY((run_pass<T, true, -1>(P, "mv_dft_d0", g.T[0], g.T[0], rows, 1, fl, NoMid(),
                          arr_store<cx<T>>(P, X1, 1, 0, g.T[0]), (double)rows * (g.n[0] * sizeof(S) + g.T[0] * e))));
   TRY((run_pass<T, false, -1>(P, "mv_dft_d1", g.T[1], g.T[1], g.T[0], g.n[2],
