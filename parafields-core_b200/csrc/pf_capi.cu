@@ -253,12 +253,14 @@ struct pf_plan {
   bool borrowed_ws = false;
   // learned preconditioner of the residual-mode CG (pf_plan_set_preconditioner), not owned
   pf_learned* learned = nullptr;
-  // autotuned choices per generation pass (0 noise, 1 middle c2c, 2 c2r): kernel family
-  // (0: paired FP32 power-of-two kernel where eligible, 1: any-length kernel) and resident CTAs per SM of persistent
-  // kernels (0: as many as fit); grid_cap is the value of the pass being launched
+  // autotuned choices per generation pass (0 noise, 1 middle c2c, 2 c2r): kernel family (0: paired
+  // FP32 kernel where the pass has one, else the any-length kernel; 1: any-length; 2: staged tiles)
+  // and resident CTAs per SM of persistent kernels (0: as many as fit); gen_pass is the pass being
+  // launched (-1: none), resident[pass] how many CTAs of its last persistent kernel fit on an SM
   int tune_variant[3] = {0, 0, 0};
   int tune_grid[3] = {0, 0, 0};
-  int grid_cap = 0;
+  int gen_pass = -1;
+  int resident[3] = {0, 0, 0};
   // pipelined batches: two streams, each with its own pair of generation workspaces
   cudaStream_t lane[2] = {nullptr, nullptr};
   cudaEvent_t lane_ev[3] = {nullptr, nullptr, nullptr};
@@ -506,7 +508,11 @@ template <typename K>
 static pf_status persistent_grid(pf_plan* P, K kern, size_t smem, long long ntiles, unsigned* grid) {
   int per = 0;
   TRY(kernel_ready(P, kern, kThreads, smem, &per));
-  if (P->grid_cap > 0 && P->grid_cap < per) per = P->grid_cap;
+  if (P->gen_pass >= 0) {
+    P->resident[P->gen_pass] = per;
+    const int cap = P->tune_grid[P->gen_pass];
+    if (cap > 0 && cap < per) per = cap;
+  }
   long long g = (long long)per * sm_count(P);
   if (g > ntiles) g = ntiles;
   *grid = (unsigned)(g > 0 ? g : 1);
@@ -981,13 +987,13 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
   // eigenvalue hit L2), the noise buffer if any, the kept output planes written once
   const double b1 = (double)g.S * lam_b + (double)T0c * outer * (Tl * noise_b + (double)g.n[last] * e);
   constexpr bool F32 = std::is_same<T, float>::value && std::is_same<S, float>::value;
-  struct CapReset {
+  struct PassReset {
     pf_plan* P;
-    ~CapReset() { P->grid_cap = 0; }
-  } cap_reset{P};
-  P->grid_cap = P->tune_grid[0];
+    ~PassReset() { P->gen_pass = -1; }
+  } pass_reset{P};
+  P->gen_pass = 0;
   if (!(stages & 1)) {
-  } else if (F32 && P->tune_variant[0] == 0 && (p2_length(Tl) || p2_length3(Tl)) && p2_view_ok(W1, jst, P0, outer))
+  } else if (F32 && P->tune_variant[0] == 0 && p2_noise_length(Tl) && p2_view_ok(W1, jst, P0, outer))
     TRY(p2_noise(P, "gen_noise_last", Tl, g.n[last], T0c, outer, nz, p2_store(P, W1, jst, P0, T0c), b1));
   else if (noise_dev)
     TRY((run_pass<T, false, +1>(P, "gen_noise_last", Tl, g.n[last], T0c, outer, R2CNoiseBuf{nz}, NoMid(),
@@ -1000,7 +1006,7 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
   // the field rows starting at `dst`
   auto c2r_rows = [&](const void* src, S* dst, long long nrows) -> pf_status {
     const double b3 = (double)nrows * (T0c * e + g.n[0] * sizeof(S));
-    P->grid_cap = P->tune_grid[2];
+    P->gen_pass = 2;
     const size_t left = (size_t)(g.domain - (size_t)(dst - out));
     if constexpr (F32) {
       if (P->tune_variant[2] == 2 && g.T[0] % 2 == 0 && p2_length(g.T[0] / 2)) {  // rows staged by bulk copies
@@ -1042,7 +1048,7 @@ static pf_status gen_r2c(pf_plan* P, const double* noise_dev, uint64_t seed, S* 
     const int nz = std::min(gp, n2 - z0);
     void* src = (char*)W1 + sizeof(cx<T>) * (size_t)w1_plane * z0;
     const double b2 = (double)T0c * nz * (g.T[1] + g.n[1]) * e;
-    P->grid_cap = P->tune_grid[1];
+    P->gen_pass = 1;
     const bool p2ok = F32 && p2_length(g.T[1]) && p2_view_ok(src, P0, w1_plane, nz) &&
                       p2_view_ok(W2, P0, w2_plane, nz);
     const P2ArrLoad l1 = p2_load(P, src, P0, w1_plane, g.T[1], T0c);
