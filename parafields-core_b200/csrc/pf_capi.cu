@@ -772,7 +772,6 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
       }
     }
   } else if (g.mb == PF_MATRIX_R2C) {
-    const bool dct = false;
     const int T0c = g.T0c;
     const long long rows = (long long)(g.N / (uint64_t)g.T[0]);
     // dimension 0: covariance evaluation fused into the R2C load
@@ -785,19 +784,19 @@ static pf_status build_spectrum(pf_plan* P, const double* vals = nullptr) {
                                    rows * T0c * 16.0)));
     spec = (double2*)A;
     if (dim >= 2) {
-      const int L1 = g.T[1], L1o = dct ? g.T[1] / 2 + 1 : g.T[1];
+      const int L1 = g.T[1];
       const long long outer = dim == 3 ? g.T[2] : 1;
-      TRY((run_pass<double, false, -1>(P, "spec_c2c_d1", L1, L1o, T0c, outer,
+      TRY((run_pass<double, false, -1>(P, "spec_c2c_d1", L1, L1, T0c, outer,
                                                    arr_load<double2>(P, A, T0c, (long long)T0c * L1, 1, L1), NoMid(),
-                                                   arr_store<double2>(P, A, T0c, (long long)T0c * L1o, 1),
-                                                   (double)T0c * outer * (L1 + L1o) * 16.0)));
+                                                   arr_store<double2>(P, A, T0c, (long long)T0c * L1, 1),
+                                                   (double)T0c * outer * 2.0 * L1 * 16.0)));
       if (dim == 3) {
-        const int L2 = g.T[2], L2o = dct ? g.T[2] / 2 + 1 : g.T[2];
-        const long long inner = (long long)T0c * L1o;
-        TRY((run_pass<double, false, -1>(P, "spec_c2c_d2", L2, L2o, inner, 1,
+        const int L2 = g.T[2];
+        const long long inner = (long long)T0c * L1;
+        TRY((run_pass<double, false, -1>(P, "spec_c2c_d2", L2, L2, inner, 1,
                                                      arr_load<double2>(P, A, inner, 0, 1, L2), NoMid(),
                                                      arr_store<double2>(P, A, inner, 0, 1),
-                                                     (double)inner * (L2 + L2o) * 16.0)));
+                                                     (double)inner * 2.0 * L2 * 16.0)));
       }
     }
   } else {  // DFT matrix: complex torus, every axis complex (dftmatrixbackend.hh:209-238)

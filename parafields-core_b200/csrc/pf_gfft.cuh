@@ -321,7 +321,7 @@ struct GArgs {
   int pitch;           // slots of one row
   int np, tpo;         // pencils (per outer block), tiles per outer block
   int args_at;         // slot of shared memory that holds a copy of these for the shared stages; 0: none
-  unsigned mL, mLh, mLout;  // divisors L, L/2, outputs per row of the post-processing
+  unsigned mL, mLout;  // divisors L, outputs per row of the post-processing
   const W* tw;         // stage twiddles
   const W* twT;        // real rows: exp(-2 pi i m / 2L), m < L
   const W* chirp;      // Bluestein: w_j, j < L
@@ -756,17 +756,9 @@ struct GNoise {
   __device__ __forceinline__ void one(unsigned i, unsigned l0, unsigned l1, int n, bool self, cx<T>& x0,
                                       cx<T>& x1) const {
     T r1, r2, r3, r4;
-    if (z.noise) {
-      const double *u = z.noise + 2 * (size_t)i, *v = u + 2 * (size_t)ss * (unsigned)h;
-      r1 = (T)u[0];
-      r2 = (T)u[1];
-      r3 = (T)v[0];
-      r4 = (T)v[1];
-    } else {
-      const uint4 c = pair_bits(z.seed, i, z.epoch ? __ldg(z.epoch) : 0u);
-      box_muller(c.x, c.y, r1, r2);
-      box_muller(c.z, c.w, r3, r4);
-    }
+    const uint4 c = pair_bits(z.seed, i, z.epoch ? __ldg(z.epoch) : 0u);
+    box_muller(c.x, c.y, r1, r2);
+    box_muller(c.z, c.w, r3, r4);
     x0 = value(l0, self && n == 0, r1, r2);
     x1 = value(l1, self && n == 0, r3, r4);
   }

@@ -165,7 +165,6 @@ static void g_fill(GArgs<T>& a, const GSched& sc, int N, int L, int Lout, int mo
   a.M1p = ROWS && M1 % 2 == 0 && (size_t)16 * (N + R1) <= kGSmem ? M1 + 1 : M1;
   a.pitch = a.M1p * R1;
   a.mL = g_magic(L);
-  a.mLh = g_magic(L / 2);
   // items per slot of the store phase
   a.mLout = g_magic(mode == 1 ? L / 2 + 1 : (mode == 2 ? (Lout + 1) / 2 : (mid ? std::min(Lout, L) : Lout)));
 }

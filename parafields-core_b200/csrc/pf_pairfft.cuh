@@ -1055,19 +1055,16 @@ __global__ void __launch_bounds__(kP2Threads, 2)
   p2_report(bad);
 }
 
-// field rows of n0 reals (row p at p * n0) of type O (FP32 fields, or the FP64 vectors of
-// the matvec and the CG), value transform applied in FP32
-template <typename O>
-struct P2FieldStoreT {
-  using O2 = typename std::conditional<sizeof(O) == 8, double2, float2>::type;
-  O* out;
+// field rows of n0 reals (row p at p * n0), value transform applied
+struct P2FieldStore {
+  float* out;
   int n0;
   int transform;
   float boxcox;
   unsigned n;
   int np;
   int Lout;
-  int vec;  // out is aligned for pairs (8 bytes FP32, 16 bytes FP64) and n0 is even
+  int vec;  // out is aligned to 8 bytes and n0 is even
   __device__ __forceinline__ void row(int p, int m, float a, float b, unsigned& bad) const {
     if (p >= np) return;
     if (transform) {
@@ -1080,13 +1077,10 @@ struct P2FieldStoreT {
     bad |= (unsigned)!ok;
     if (!ok) return;
     if (two && vec) {
-      O2 v;
-      v.x = (O)a;
-      v.y = (O)b;
-      *reinterpret_cast<O2*>(out + i) = v;
+      *reinterpret_cast<float2*>(out + i) = make_float2(a, b);
     } else {
-      out[i] = (O)a;
-      if (two) out[i + 1] = (O)b;
+      out[i] = a;
+      if (two) out[i + 1] = b;
     }
   }
   __device__ __forceinline__ void store(int p, int m, const P2& z, unsigned& bad) const {
@@ -1094,7 +1088,6 @@ struct P2FieldStoreT {
     row(p + 1, m, z.re.y, z.im.y, bad);
   }
 };
-using P2FieldStore = P2FieldStoreT<float>;
 
 // ---------------------------------------------------------------------------
 // Real-to-complex rows (L+1 complex from 2L reals, FFTW r2c semantics), the forward
