@@ -414,10 +414,11 @@ pf_status pf_plan_set_preconditioner(pf_plan* plan, pf_learned* learned);
 /* Measured planning, the counterpart of fftw.measure / fftw.useWisdom (r2cfieldbackend.hh:
  * 212-230, fieldtraits.hh:175-186): times every candidate of each realization pass of the
  * plan (the kernels that the pass has -- any-length always, paired or staged FP32 ones at
- * some lengths -- x resident CTAs per SM of the persistent ones, `repetitions` realizations
- * each, default 3; a pass with one candidate is not timed) and keeps the fastest per pass (a
- * pass whose paired and any-length kernels come within 10% is decided on a batch); then, on batches of 4
- * realizations, the plane groups of the last two 3D passes and the batch mode of
+ * some lengths -- x resident CTAs per SM of the persistent ones, the fastest of `repetitions`
+ * realizations each, at least and by default 3; a pass with one candidate is not timed) and
+ * keeps the fastest per pass (staged kernels have to gain 3% and run faster on a batch; a
+ * pass whose paired and any-length kernels come within 10% is decided on a batch); then, on
+ * batches of 4 realizations, the plane groups of the last two 3D passes and the batch mode of
  * pf_generate_batch.  Choices go to
  * a process-wide wisdom table keyed by the pass geometry; a plan whose passes are all in it
  * takes them without timing (*timed = 0).  Clears the plan's profiling records.  R2C field

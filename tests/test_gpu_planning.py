@@ -59,6 +59,22 @@ def test_rows_have_no_paired_kernel():
         assert wisdom[2] == (0, 0) or wisdom[2][0] == 2
 
 
+def test_repeated_plannings_agree():
+    """256^3 FP32: 256-point rows staged by bulk copies take 72 us, the any-length ones 70, in events
+    that resolve 2 us; forty plannings of one repetition all keep the latter"""
+    plan = pfb200.Plan(pfb200.make_desc(dim=3, cells=(256, 256, 256), covariance="matern32", corr_length=0.1,
+                                        approximate=True, precision=F32))
+    plan.spectrum_build()
+    seen = set()
+    for _ in range(40):
+        pfb200.wisdom_forget()
+        plan.autotune(repetitions=1)
+        seen |= {line.split()[5] for line in pfb200.wisdom_export().strip().splitlines() if line.split()[0] == "2"}
+    pfb200.wisdom_forget()
+    plan.close()
+    assert seen == {"0"}
+
+
 @pytest.mark.parametrize("cells,precision", [((128, 128, 64), F32), ((192, 96, 192), F32), ((64, 48), F64)])
 def test_planned_fields_equal_unplanned_ones(cells, precision):
     """to the rounding of the kernels that planning may exchange: FP32 1e-5 (eps 6e-8 times a few
