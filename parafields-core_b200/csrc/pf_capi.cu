@@ -490,8 +490,6 @@ static size_t cap_of(const pf_plan* P, const void* p) {
   return 0;
 }
 
-// compile-time specialised passes for the common lengths; other lengths fall back to
-// the runtime-radix kernels above
 static int sm_count(pf_plan* P) {
   static int cached[128] = {0};
   const int d = P->device < 128 ? P->device : 0;
@@ -1200,8 +1198,8 @@ static pf_status matvec_r2c(pf_plan* P, int op, const S* in, S* out) {
   const int row_pairs_out = g.n[0] % 2 == 0 && ((uintptr_t)out % (2 * sizeof(S))) == 0;
   FieldRowLoad<S> fl{in, g.n[0], (unsigned)g.domain, row_pairs_in};
   FieldRowStore<S> fs{out, g.n[0], 0, 0.0, (unsigned)g.domain, row_pairs_out};
-  // the real-to-complex and complex-to-real rows along dim 0 take the paired kernels where
-  // T0/2 is a power of two in [128, 2048] (FP32 transforms)
+  // the real-to-complex rows along dim 0 take the paired kernel where T0/2 is a power of two in
+  // [128, 2048] (FP32 transforms); the complex-to-real rows run on the any-length kernel
   const bool p2rows = std::is_same<T, float>::value && g.T[0] % 2 == 0 && p2_length(g.T[0] / 2);
   const int pair_ok = (g.n[0] % 2 == 0) ? 1 : 0;
   auto fwd_rows = [&](void* X, long long nrows) -> pf_status {

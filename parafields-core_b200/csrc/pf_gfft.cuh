@@ -28,8 +28,11 @@
 // w_j = exp(-pi i j^2 / L), X_k = w_k sum_j (x_j w_j) conj(w_(k-j)), a circular convolution of
 // the cheapest smooth length N >= 2 L - 1.
 //
-// What bounds it: latency -- of loads, barriers and instruction fetch -- at 16-32 warps per SM; the
-// issue slots are 35-55% busy, HBM below 45%.  Measured on one B200 against the passes it replaced
+// What bounds it: latency -- of loads, barriers and instruction fetch -- at 25-30 warps per SM; the
+// issue slots are 29-45% busy in FP64 strided passes, rows and covariance rows (100^3 field, 128 x 120
+// x 96 spectrum; FP64 pipe 13-22%), 59% in the FP32 fused pass (128^3) and 69% in the FP64 noise pass
+// (100^3; FP64 pipe 39%), which issue bounds most.  The loaders' long scoreboard is the first
+// stall of all others; covariance rows add spills (868 bytes stored, 64 registers).  Measured on one B200 against the passes it replaced
 // (two ping-pong buffers, runtime divisions per element, 2 CTAs per SM; compile-time schedules
 // for 11 lengths; radix-2 Bluestein), us: 100^3 FP64 realization, passes of 200, 200 and 100
 // points, 116 / 44 / 34 -> 67 / 21 / 17; FP64 product on 128^3 (256 points) 287 -> 193, its fused

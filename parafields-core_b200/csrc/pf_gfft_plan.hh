@@ -97,11 +97,13 @@ constexpr size_t kGSmem = 227 * 1024;
 
 // Slots per tile and threads.  Strided tiles take 8 slots (128-byte row segments) while three
 // of them fit on an SM, fewer for longer pencils but at least 2 (one 32-byte sector) while two
-// fit; row tiles up to 1024 elements, 2048 where the loader computes its values (192-point FP32 rows
-// beside another stream's passes 87 us with 8 pairs per tile, 74 with 4; 128-point rows 15 with 8, 18 with 4).  Fewer slots
-// where the grid would leave SMs idle.  Threads: the count with the least estimated time, which
-// is rounds of butterflies (and of loader pairs) per tile over the tiles that run at once on an SM
-// within 1024 threads, the tile's shared memory and the grid.
+// fit; row tiles up to 1024 elements, 2048 where the loader computes its values (complex-to-real rows
+// of n0 x 96 x 80 fields at 17 lengths 32..512, tiles of 1024 against 2048 elements, us: FP32 192
+// points 11.6 against 13.0, 256 13.1 / 14.5, 384 21.9 / 23.1, FP64 250 27.4 / 29.3, 500 46 / 50; the
+// others within 3%, but 400 points 25.2 / 24.7 and 40.8 / 36.4; 192-point FP32 rows beside another
+// stream's passes 74 / 87).  Fewer slots where the grid would leave SMs idle.  Threads: the count
+// with the least estimated time, which is rounds of butterflies (and of loader pairs) per tile over
+// the tiles that run at once on an SM within 1024 threads, the tile's shared memory and the grid.
 static void g_tile(int slots, const std::vector<int>& r, bool rows, bool direct, int pitch, long long nslots,
                    long long nouter, int sms, int* B_out, int* nt_out) {
   const size_t per = (size_t)16 * pitch;

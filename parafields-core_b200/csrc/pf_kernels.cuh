@@ -61,7 +61,7 @@ struct NoMid {
 // Generic complex pencil pass.  CONTIG: pencils are rows (element j of row p at
 // stride 1); otherwise pencil p of outer block o has element j at p + j*jstride +
 // o*ostride, and one tile holds B consecutive p so every row segment is coalesced.
-// Registers are capped for two resident CTAs per SM (the Bluestein tiles allow two).
+// Registers are capped for two resident CTAs per SM.
 template <typename T, bool CONTIG, class Ld, class Mid, class St>
 __global__ void __launch_bounds__(kThreads, 2) k_pass(const PassArgs a, const cx<T>* __restrict__ tw,
                                                       Ld ld, Mid mid, St st) {
@@ -985,7 +985,9 @@ struct R2CNoise {
     const bool selfconj = (k0 == 0 || 2 * k0 == ext[0]) && (a1 == 0 || 2 * a1 == ext[1]) &&
                           (dim < 3 || a2 == 0 || 2 * a2 == ext[2]);
     if (selfconj) return mk<T>(lam * r1, (T)0);
-    // FP64 keeps the reference's lambda / sqrt(2) (r2cfieldbackend.hh:322-323)
+    // FP64 keeps the reference's lambda / sqrt(2) (r2cfieldbackend.hh:322-323).  The any-length
+    // kernels' seeded noise of even lengths and their noise buffers form it as a product with
+    // 1/sqrt(2) held in two doubles (GNoise::value): this quotient but for rare last digits.
     const T s = sizeof(T) == 8 ? lam / (T)1.41421356237309504880168872420969808
                                : lam * (T)0.70710678118654752440084436210484903928;
     return mk<T>(s * r1, s * r2);

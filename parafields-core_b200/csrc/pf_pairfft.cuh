@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(kP2Threads, 2)
 // in memory (row stride `rowstride` complex, 16-byte multiple), so one cp.async.bulk per
 // tile moves them into shared memory, completion counted on an mbarrier; two tile buffers
 // alternate over the persistent loop, so the next tile's copy runs while the current one
-// is transformed, and each input element is read from HBM once (the scalar kernel reads X[m]
+// is transformed, and each input element is read from HBM once (the any-length kernel reads X[m]
 // and X[L-m] as separate loads).  Rows beyond the last row read as zero; a copy whose rows
 // would leave the buffer is not issued (bit 1 of the error word, zero rows).  Every wait is
 // bounded: a wait that gives up sets bit 2 and the CTA leaves the loop (all threads together).

@@ -3,9 +3,9 @@ command line instead of measured planning, so that a profiler sees only the FP64
 and the realization passes of each choice, in order.
 
 Each `--run` is one plan: a list of PASS=VARIANT[:CTAS] entries (pass 0 noise, 1 middle
-strided, 2 complex-to-real; variant 0 paired FP32, 1 scalar, 2 staged tiles -- TMA for pass 1,
-bulk copies for pass 2; CTAS resident CTAs per SM, 0 = as many as fit) and optionally
-G=<plane groups>.  Passes not named take variant 0 at full occupancy.
+strided, 2 complex-to-real; variant 0 paired FP32 where the pass has it, 1 any-length,
+2 staged tiles -- TMA for pass 1, bulk copies for pass 2; CTAS resident CTAs per SM of the
+persistent kernels, 0 = as many as fit) and optionally G=<plane groups>.  Passes not named take variant 0 at full occupancy.
 
   python parafields-core_b200/pass_profile.py --cells 256 256 256 --covariance matern32 \\
       --corr-length 0.2 0.1 0.05 --approximate --run 2=0 --run 2=2 --realizations 2
